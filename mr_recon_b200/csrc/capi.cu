@@ -119,7 +119,7 @@ int mrn_sense_normal(mrn_plan* P, const void* x, const void* mps, const float* d
     // density weight applied by the interpolation (the same products, so the
     // same bits as the sample-order path)
     const EntIO eio{P->d_ent_of, dcf, P->max_coil, 0};
-    { StageTimer t(P, kStageInterp, ST(s)); RK(launch_interp_reg(P, P->d_grid, kInternal, P->d_ksp_ent, inv_wd(P), nullptr, ST(s), eio)); }
+    { StageTimer t(P, kStageInterp, ST(s)); RK(gather_ok(P, kInternal) ? launch_interp_gather(P, P->d_grid, kInternal, P->d_ksp_ent, inv_wd(P), ST(s), eio) : launch_interp_reg(P, P->d_grid, kInternal, P->d_ksp_ent, inv_wd(P), nullptr, ST(s), eio)); }
     {
       StageTimer t(P, kStageGrid, ST(s));
       if (P->n_items_grid > 0) {

@@ -45,7 +45,24 @@ struct SliceGeom {
   float inv_sqrt_n;      // 1 / sqrt(prod(n)) (fourier.py:462, 522)
   int native_fft;        // the slice's FFT group runs the native passes (ffx.cu),
                          // which pad and crop it themselves
+  int cb;                // coils per block of the internal grid: [coil block][cell][cb] (1: coil planes)
 };
+
+// Coils per block of a slice's internal grid: 8 (64 bytes a cell), or the next
+// power of two for fewer coils. Interpolation at 128^3, 16 coils, 2.05 M
+// kooshball samples, W 4: blocks of 16 / 8 / 4 coils 1.13 / 0.99 / 1.38 ms.
+__host__ __device__ __forceinline__ int coil_block(int ncoil) {
+  return ncoil <= 2 ? ncoil : (ncoil <= 4 ? 4 : 8);
+}
+
+// Internal grid offset of (coil c, cell) within a slice: coils come in blocks
+// of cb, the cb values of one cell side by side, so a warp whose lanes are
+// coils reads or writes whole sectors of a cell. A grid of coil planes is
+// the case cb = 1 (caller grids, and grids that cuFFT transforms).
+__host__ __device__ __forceinline__ int64_t grid_at(int64_t gos, int cb, int c, int64_t cell) {
+  const int lg = cb >= 8 ? 3 : (cb >= 4 ? 2 : cb - 1);  // cb is 1, 2, 4 or 8
+  return ((((int64_t)(c >> lg)) * gos + cell) << lg) + (c & (cb - 1));
+}
 
 // Work item: one tile (or a chunk of a heavy tile) of one slice. Item lists
 // are launched at a capacity fixed when the trajectory is bound; entries past
@@ -90,17 +107,18 @@ struct EntIO {
 constexpr int kKBTerms = 32;  // terms of the I0 power series kept in KBParams
 
 // One axis of the native FFT (ffx.cu): length n = radix[0] * ... *
-// radix[ns - 1], each radix 2, 3, 4, 5, 8 or 16; stage s reads its twiddles
+// radix[ns - 1], at least two stages (the last may be 1), each radix at most 20; stage s reads its twiddles
 // exp(-2 pi i t j / (L R)), j < L = radix[0] * ... * radix[s - 1], 1 <= t < R,
 // at tw + tw_off[s] + j (R - 1) + t - 1 of the axis' table (n - 1 entries).
-constexpr int kFfxMaxStages = 12;
+constexpr int kFfxMaxStages = 4;
 constexpr int kFfxMaxN = 1024;
 struct FfxAxis {
   int n;
   int ns;
   int radix[kFfxMaxStages];
   int tw_off[kFfxMaxStages];
-  unsigned magic[kFfxMaxStages];  // floor(2^32 / L) + 1: b / L = umulhi(b, magic) for b, L <= kFfxMaxN
+  unsigned mag_l[kFfxMaxStages];   // floor(2^32 / L) + 1: b / L = umulhi(b, mag_l) for b < 2^16
+  unsigned mag_nr[kFfxMaxStages];  // the same for n / radix
   int tw_base;  // first entry of this axis in the plan's twiddle table
 };
 
@@ -113,28 +131,23 @@ struct FfxGroup {
   int first_slice;  // geometry (image and grid size) shared by the group's slices
   int nsl;          // slices in the group
   int sl_off;       // their ids at FfxSet::d_sl + sl_off, in grid order
-  int row_off;      // first grid row of each at FfxSet::d_row + row_off (nsl + 1 entries)
-  int64_t nrows;    // grid rows (coils x all axes but the last) of the group
-  int64_t grid_off; // complex offset of the group's block in its grid buffer
-  int batch;        // coils of the group
+  int max_coil;     // coils of the widest slice, padded to whole coil blocks
+  int total_coil;   // padded coils of all slices
 };
 
 // The native FFT of one grid buffer: its groups, their twiddle tables and
-// slice / row lists (host side owns the device arrays; release() frees them).
+// slice lists (host side owns the device arrays; release() frees them).
 struct FfxSet {
   bool ok = false;   // some group is native
   bool all = false;  // every group is native
   std::vector<FfxGroup> grp;
   float2* d_tw = nullptr;
   int* d_sl = nullptr;
-  int64_t* d_row = nullptr;
   void release() {
     if (d_tw) cudaFree(d_tw);
     if (d_sl) cudaFree(d_sl);
-    if (d_row) cudaFree(d_row);
     d_tw = nullptr;
     d_sl = nullptr;
-    d_row = nullptr;
     grp.clear();
     ok = all = false;
   }
@@ -381,6 +394,7 @@ struct mrn_plan {
   mrn::KBParams kb{};
   std::vector<mrn::SliceGeom> h_slices;
   int64_t n_img = 0, n_ksp = 0, n_grid = 0, n_trj = 0, n_pts = 0, n_x = 0;
+  int64_t n_igrid = 0;  // elements of d_grid (whole coil blocks)
   int64_t n_prow = 0, n_irow = 0, n_xrow = 0;  // row counts of the grid / image layouts
   int ntiles = 0;   // interpolation tiles, all slices
   int ngtiles = 0;  // gridding tiles, all slices
@@ -470,6 +484,17 @@ struct mrn_plan {
   // selects it (default) or cuFFT for every group.
   mrn::FfxSet ffx;
   bool use_ffx = true;
+  // Interpolation from the grid in coil blocks (gather.cu): the slices of
+  // each block width, cut into CTAs of `chunk` sorted samples.
+  struct GatherSet {
+    int cb;        // coils per block of these slices
+    int nsl;       // slices
+    int chunk;     // samples per CTA
+    int nchunks;   // CTAs
+    int off;       // slice ids at d_gather + off, then their first CTAs (nsl + 1 entries)
+  };
+  std::vector<GatherSet> gather;
+  int* d_gather = nullptr;
 
   // Optional stage timing (mrn_plan_enable_timing): CUDA event pairs recorded
   // on the launching stream around each stage, summed by mrn_plan_timing.

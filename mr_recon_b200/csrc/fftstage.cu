@@ -172,7 +172,7 @@ __device__ __forceinline__ void post_row(const SliceGeom* __restrict__ sl, int n
       float ax = 0.f, ay = 0.f;
 #pragma unroll 4
       for (int c = 0; c < g.ncoil; ++c) {
-        const float2 y = grid[g.grid_off + (int64_t)c * g.gos + slin + sj];
+        const float2 y = grid[g.grid_off + grid_at(g.gos, g.cb, c, slin + sj)];
         const float2 m = __ldg(mps + g.img_off + (int64_t)c * g.nimg + orow * nl + j);
         // conj(m) * y
         ax += m.x * y.x + m.y * y.y;
@@ -195,36 +195,47 @@ __device__ __forceinline__ void post_row(const SliceGeom* __restrict__ sl, int n
   }
 }
 
-// Copy between the caller's centred grid layout (slice order) and the
-// internal natural-order layout (FFT groups): centred k <-> storage (k - Nos//2) mod Nos.
+// Copy between the caller's centred grid layout (slice order, coil planes) and
+// the internal one: coil blocks in the same cell order (native slices), or
+// coil planes in FFT order, centred k <-> storage (k - Nos//2) mod Nos. One
+// thread per cell of one coil block: it moves the block's cb values, which
+// are contiguous inside, while adjacent threads take adjacent cells of each
+// of the caller's planes.
 template <int D>
-__global__ void k_shift_copy(const SliceGeom* __restrict__ sl, int ns, const float2* __restrict__ src,
-                             float2* __restrict__ dst, int to_user, int64_t total) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= total) return;
-  int lo = 0, hi = ns - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (sl[mid].ugrid_off <= idx) lo = mid; else hi = mid - 1;
+__global__ void __launch_bounds__(256)
+k_shift_copy(const SliceGeom* __restrict__ sl, int ns, const float2* __restrict__ src, float2* __restrict__ dst,
+             int to_user) {
+  const int64_t cell = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int s = blockIdx.z; s < ns; s += gridDim.z) {
+    const SliceGeom& g = sl[s];
+    if (cell >= g.gos) continue;
+    int64_t scell = cell;
+    if (!g.native_fft) {
+      int64_t r = cell;
+      int k[kMaxDim] = {0, 0, 0};
+      for (int i = D - 1; i >= 0; --i) {
+        k[i] = (int)(r % g.nos[i]);
+        r /= g.nos[i];
+      }
+      scell = 0;
+      for (int i = 0; i < D; ++i) {
+        int t = k[i] - g.hshift[i];
+        if (t < 0) t += g.nos[i];
+        scell = scell * g.nos[i] + t;
+      }
+    }
+    const int cb = g.cb;
+    for (int c0 = blockIdx.y * cb; c0 < g.ncoil; c0 += gridDim.y * cb) {
+      const int nc = min(cb, g.ncoil - c0);
+      const int64_t in = g.grid_off + grid_at(g.gos, cb, c0, scell);
+      const int64_t us = g.ugrid_off + (int64_t)c0 * g.gos + cell;
+#pragma unroll 8
+      for (int c = 0; c < nc; ++c) {
+        if (to_user) dst[us + c * g.gos] = src[in + c];
+        else dst[in + c] = src[us + c * g.gos];
+      }
+    }
   }
-  const SliceGeom& g = sl[lo];
-  const int64_t r = idx - g.ugrid_off;
-  const int64_t c = r / g.gos;
-  int64_t cell = r - c * g.gos;
-  int k[kMaxDim] = {0, 0, 0};
-  for (int i = D - 1; i >= 0; --i) {
-    k[i] = (int)(cell % g.nos[i]);
-    cell /= g.nos[i];
-  }
-  int64_t slin = 0;
-  for (int i = 0; i < D; ++i) {
-    int s = k[i] - g.hshift[i];
-    if (s < 0) s += g.nos[i];
-    slin = slin * g.nos[i] + s;
-  }
-  const int64_t ii = g.grid_off + c * g.gos + slin;
-  if (to_user) dst[idx] = src[ii];
-  else dst[ii] = src[idx];
 }
 
 int launch_pre(mrn_plan* P, PreMode mode, const float2* src, const float2* mps, float scale,
@@ -270,14 +281,18 @@ k_post_sense(const SliceGeom* __restrict__ sl, int ns, const float* __restrict__
   }
   for (int i = 0; i < D - 1; ++i) {
     aout *= apod[g.apod_off[i] + q[i]];
-    int sidx = q[i] - g.n[i] / 2;
-    if (sidx < 0) sidx += g.nos[i];
+    int sidx = q[i];
+    if (!g.native_fft) {
+      sidx -= g.n[i] / 2;
+      if (sidx < 0) sidx += g.nos[i];
+    }
     slin = slin * g.nos[i] + sidx;
   }
-  const int nl = g.n[D - 1], nosl = g.nos[D - 1], h = nl / 2;
+  // the native passes leave image point q in row q of every axis
+  const int nl = g.n[D - 1], nosl = g.nos[D - 1], h = g.native_fft ? 0 : nl / 2, cb = g.cb;
   slin *= nosl;
   const float* al = apod + g.apod_off[D - 1];
-  const float2* gbase = grid + g.grid_off + slin;
+  const float2* gbase = grid + g.grid_off;
   const float2* mbase = mps + g.img_off + orow * nl;
   float2* orow_p = out + g.x_off + orow * nl;
   const float2* xrow = xin ? xin + g.x_off + orow * nl : nullptr;
@@ -288,7 +303,7 @@ k_post_sense(const SliceGeom* __restrict__ sl, int ns, const float* __restrict__
     float ax = 0.f, ay = 0.f;
 #pragma unroll 8
     for (int c = 0; c < g.ncoil; ++c) {
-      const float2 y = gbase[(int64_t)c * g.gos + sj];
+      const float2 y = gbase[grid_at(g.gos, cb, c, slin + sj)];
       const float2 m = __ldg(mbase + (int64_t)c * g.nimg + j);
       // conj(m) * y
       ax += m.x * y.x + m.y * y.y;
@@ -356,15 +371,18 @@ int launch_post(mrn_plan* P, PostMode mode, const float2* mps, float2* out, floa
 }
 
 int launch_shift_copy(mrn_plan* P, const float2* src, float2* dst, int to_user, cudaStream_t st) {
-  const int64_t total = P->n_grid;
-  const unsigned blocks = (unsigned)((total + 255) / 256);
-  if (blocks == 0) return MRN_OK;
-  if (P->ndim == 1)
-    k_shift_copy<1><<<blocks, 256, 0, st>>>(P->d_slices, P->nslices, src, dst, to_user, total);
-  else if (P->ndim == 2)
-    k_shift_copy<2><<<blocks, 256, 0, st>>>(P->d_slices, P->nslices, src, dst, to_user, total);
-  else
-    k_shift_copy<3><<<blocks, 256, 0, st>>>(P->d_slices, P->nslices, src, dst, to_user, total);
+  int64_t cells = 0;
+  int blocks = 1;
+  for (const SliceGeom& g : P->h_slices) {
+    cells = std::max(cells, g.gos);
+    blocks = std::max(blocks, (g.ncoil + g.cb - 1) / g.cb);
+  }
+  if ((cells + 255) / 256 > 0x7fffffffLL) return MRN_ERR_UNSUPPORTED;
+  const dim3 gd((unsigned)((cells + 255) / 256), (unsigned)std::min(blocks, 65535),
+                (unsigned)std::min(P->nslices, 65535));
+  if (P->ndim == 1) k_shift_copy<1><<<gd, 256, 0, st>>>(P->d_slices, P->nslices, src, dst, to_user);
+  else if (P->ndim == 2) k_shift_copy<2><<<gd, 256, 0, st>>>(P->d_slices, P->nslices, src, dst, to_user);
+  else k_shift_copy<3><<<gd, 256, 0, st>>>(P->d_slices, P->nslices, src, dst, to_user);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? MRN_OK : cuda_fail(e);
 }
@@ -406,6 +424,20 @@ int inv_transform(mrn_plan* P, float2* out, cudaStream_t st) {
   if (!out) return MRN_OK;
   StageTimer t(P, kStagePost, st);
   return launch_post(P, kPostPlain, nullptr, out, 1.0f, nullptr, 0.f, nullptr, 0, st);
+}
+
+int cufft_setup(mrn_plan* P) {
+  for (size_t q = 0; q < P->fft.size(); ++q) {
+    auto& fg = P->fft[q];
+    if (fg.handle || (P->use_ffx && q < P->ffx.grp.size() && P->ffx.grp[q].native)) continue;
+    int n[kMaxDim];
+    for (int i = 0; i < P->ndim; ++i) n[i] = fg.nos[i];
+    if (cufftPlanMany(&fg.handle, P->ndim, n, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C, fg.batch) != CUFFT_SUCCESS) {
+      fg.handle = 0;
+      return MRN_ERR_CUFFT;
+    }
+  }
+  return MRN_OK;
 }
 
 int run_fft(mrn_plan* P, int direction, cudaStream_t st, bool skip_native) {

@@ -328,7 +328,8 @@ k_grid_reg3(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KB
   const int hs0 = layout == kInternal ? gp->hshift[0] : 0;
   const int hs1 = layout == kInternal ? gp->hshift[1] : 0;
   const int hs2 = layout == kInternal ? gp->hshift[2] : 0;
-  float2* dst = grid + (layout == kInternal ? gp->grid_off : gp->ugrid_off) + (int64_t)c0 * gp->gos;
+  float2* dst = grid + (layout == kInternal ? gp->grid_off : gp->ugrid_off);
+  const int cb = layout == kInternal ? gp->cb : 1;
   // this thread's cell of every block it stores: (y, z) fixed, block varies
   const int cell = tid & 63, cy = cell >> 3, cz = cell & 7;
   const bool cell_in = cy < f.size[1] && cz < f.size[2];
@@ -355,7 +356,7 @@ k_grid_reg3(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KB
         *split_slot(so, it.split, c0 + bc, (bp * f.size[1] + cy) * f.size[2] + cz) = val;
       } else {
         const int64_t xo = (int64_t)wrap_once(f.org[0] + bp - hs0, nos0) * nos1 * nos2;
-        dst[(int64_t)bc * gp->gos + xo + yz] = val;
+        dst[grid_at(gp->gos, cb, c0 + bc, xo + yz)] = val;
       }
     }
   }

@@ -60,6 +60,11 @@ int launch_interp_reg(mrn_plan* P, const float2* grid, int layout, float2* ksp, 
                       const float2* temporal, cudaStream_t st, EntIO eio = EntIO{nullptr, nullptr, 0, 0});
 int launch_trajgrad_reg(mrn_plan* P, const float2* grid, int layout, const float2* samples, float* out,
                         float scale, cudaStream_t st);
+// Interpolation straight from a grid in coil blocks (gather.cu)
+int gather_setup(mrn_plan* P);
+bool gather_ok(const mrn_plan* P, int layout);
+int launch_interp_gather(mrn_plan* P, const float2* grid, int layout, float2* ksp, float scale, cudaStream_t st,
+                         EntIO eio = EntIO{nullptr, nullptr, 0, 0});
 bool grid_reg_ok(const mrn_plan* P);
 bool grid_reg3_ok(const mrn_plan* P);
 int launch_grid_reg3(mrn_plan* P, const float2* ksp, const float* dcf, const float2* temporal,
@@ -93,6 +98,9 @@ int launch_shift_copy(mrn_plan* P, const float2* src, float2* dst, int to_user, 
 // cuFFT of every FFT group, or (skip_native) of the groups the native passes
 // do not cover.
 int run_fft(mrn_plan* P, int direction, cudaStream_t st, bool skip_native = false);
+// cuFFT plans of the groups that need one: those the native passes do not
+// cover, every group once MRN_OPT_NATIVE_FFT is 0.
+int cufft_setup(mrn_plan* P);
 // Apodize / pad and forward FFT of the plan grid (native passes when
 // ffx_active, else k_pre + cuFFT), stage-timed; and the inverse FFT with the
 // plain crop / deapodize into out, or (out == nullptr) leaving the grid for a
@@ -104,13 +112,11 @@ int inv_transform(mrn_plan* P, float2* out, cudaStream_t st);
 // Slice table upload (plan.cu): d_slices and its shared-k-space twin.
 cudaError_t upload_slices(mrn_plan* P);
 
-// Native FFT (ffx.cu). A grid buffer of FFT groups: per group its grid size,
-// the offset of its [batch][nos...] block and its coils; FfxGrid is what the
-// passes read (host and device slice tables, apodization, the buffer).
+// Native FFT (ffx.cu). A grid buffer of FFT groups, each one grid size;
+// FfxGrid is what the passes read (host and device slice tables,
+// apodization, the buffer).
 struct FfxGroupSpec {
   int nos[kMaxDim];
-  int64_t grid_off;
-  int batch;
 };
 struct FfxGrid {
   int ndim;
@@ -118,7 +124,9 @@ struct FfxGrid {
   const SliceGeom* dsl;
   const float* apod;
   float2* grid;
+  int sm_count;
 };
+bool ffx_can(int ndim, const int* nos);  // every axis of the grid size can run natively
 int ffx_build(FfxSet& S, int ndim, const std::vector<SliceGeom>& hsl, const std::vector<FfxGroupSpec>& spec);
 int ffx_fwd(const FfxSet& S, const FfxGrid& G, PreMode mode, const float2* src, const float2* mps, float scale,
             cudaStream_t st);

@@ -608,20 +608,28 @@ int mrn_plan_create(mrn_plan** out, int ndim, int n_slices, const int* im_size,
         found = (int)P->fft.size() - 1;
       }
       group_of[s] = found;
-      P->fft[found].batch += g.ncoil;
     }
+    // grids that can run the native passes hold whole coil blocks; with
+    // MRN_OPT_NATIVE_FFT 0 their unused coils are transformed along
     int64_t off = 0;
     for (size_t q = 0; q < P->fft.size(); ++q) {
       P->fft[q].grid_off = off;
+      const bool can = ffx_can(ndim, P->fft[q].nos);
       for (int s = 0; s < n_slices; ++s)
         if (group_of[s] == (int)q) {
-          P->h_slices[s].grid_off = off;
-          off += (int64_t)P->h_slices[s].ncoil * P->h_slices[s].gos;
+          SliceGeom& g = P->h_slices[s];
+          const int cb = can ? coil_block(g.ncoil) : 1;
+          const int padded = (g.ncoil + cb - 1) / cb * cb;
+          g.grid_off = off;
+          off += (int64_t)padded * g.gos;
+          P->fft[q].batch += padded;
         }
     }
+    P->n_igrid = off;
   } else {
     for (int s = 0; s < n_slices; ++s) P->h_slices[s].grid_off = P->h_slices[s].ugrid_off;
   }
+  for (auto& g : P->h_slices) g.cb = 1;  // ffx_refresh sets the native slices' block
 
   cudaError_t e = cudaSetDevice(device);
   if (e != cudaSuccess) { delete P; return cuda_fail(e); }
@@ -682,17 +690,12 @@ int mrn_plan_create(mrn_plan** out, int ndim, int n_slices, const int* im_size,
   PK(dev_alloc(&P->d_red, (size_t)n_slices * kMaxRedBlocks));
   PK(dev_alloc(&P->d_rowpart, (size_t)std::max<int64_t>(P->n_xrow, 1)));
   if (!raw) {
-    PK(dev_alloc(&P->d_grid, std::max<int64_t>(P->n_grid, 1)));
+    PK(dev_alloc(&P->d_grid, std::max<int64_t>(P->n_igrid, 1)));
     PK(dev_alloc(&P->d_ksp_tmp, std::max<int64_t>(P->n_ksp, 1)));
-    for (auto& fg : P->fft) {
-      int n[kMaxDim];
-      for (int i = 0; i < ndim; ++i) n[i] = fg.nos[i];
-      cufftResult r = cufftPlanMany(&fg.handle, ndim, n, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C,
-                                    fg.batch);
-      if (r != CUFFT_SUCCESS) { fg.handle = 0; mrn_plan_destroy(P); return MRN_ERR_CUFFT; }
-    }
     PK(ffx_setup(P));
+    PK(cufft_setup(P));
   }
+  PK(gather_setup(P));
 #undef PK
   *out = P;
   return MRN_OK;
@@ -723,7 +726,10 @@ int mrn_plan_set_option(mrn_plan* P, int option, int value) {
       return MRN_OK;
     case MRN_OPT_NATIVE_FFT:
       P->use_ffx = value != 0;
-      return ffx_refresh(P);
+      {
+        const int rc = ffx_refresh(P);
+        return rc == MRN_OK ? cufft_setup(P) : rc;
+      }
     case MRN_OPT_GRID_LANES:
       if (value != 0 && value != 8 && value != 16 && value != 32) return MRN_ERR_ARG;
       P->grid_lanes = value;
@@ -784,7 +790,7 @@ int mrn_plan_destroy(mrn_plan* P) {
                   P->d_ksp_tmp, P->d_sync, P->d_wmeta_i, P->d_wtab_i, P->d_wmeta_g,
                   P->d_wtab_g, P->d_part, P->d_items_tmp, P->d_sort_key[0], P->d_sort_key[1],
                   P->d_sort_idx[0], P->d_sort_idx[1], P->d_red, P->d_rowpart, P->d_ent_of,
-                  P->d_ksp_ent};
+                  P->d_ksp_ent, P->d_gather};
   for (void* b : bufs)
     if (b) cudaFree(b);
   delete P;

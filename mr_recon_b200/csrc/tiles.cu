@@ -63,7 +63,7 @@ __device__ __forceinline__ float coord_of(const float4& c, int i) {
 // into shared memory [c][cells] with plane stride pstride. One warp per row.
 template <int D>
 __device__ __forceinline__ void load_region(float2* __restrict__ tile, const float2* __restrict__ grid,
-                                            int64_t goff, int64_t gos, const SliceGeom& g,
+                                            int64_t goff, int64_t gos, int cb, int c0, const SliceGeom& g,
                                             const int* org, const int* ext, const int* hs, int ncg,
                                             int pstride) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -89,12 +89,12 @@ __device__ __forceinline__ void load_region(float2* __restrict__ tile, const flo
     }
     base *= g.nos[D - 1];
     lbase *= inner;
-    const float2* src = grid + goff + (int64_t)c * gos + base;
+    const float2* src = grid + goff + grid_at(gos, cb, c0 + c, base);
     float2* dst = tile + c * pstride + lbase;
     const int n = g.nos[D - 1];
     for (int q = lane; q < inner; q += 32) {
       const int s = pos_mod(org[D - 1] + q - hs[D - 1], n);
-      dst[q] = __ldg(src + s);
+      dst[q] = __ldg(src + (int64_t)s * cb);
     }
   }
 }
@@ -127,8 +127,9 @@ k_interp(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KBPar
     ext[i] = i < D ? f.size[i] + kb.ntaps[i] - 1 : 1;
     hs[i] = (i < D && layout == kInternal) ? g.hshift[i] : 0;
   }
-  const int64_t goff = (layout == kInternal ? g.grid_off : g.ugrid_off) + (int64_t)c0 * g.gos;
-  load_region<D>(tile, grid, goff, g.gos, g, f.org, ext, hs, ncg, pstride);
+  const int64_t goff = layout == kInternal ? g.grid_off : g.ugrid_off;
+  const int cb = layout == kInternal ? g.cb : 1;
+  load_region<D>(tile, grid, goff, g.gos, cb, c0, g, f.org, ext, hs, ncg, pstride);
   __syncthreads();
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -424,7 +425,8 @@ k_grid(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KBParam
   // write-back: one store per cell (into the item's partial slot for split tiles)
   int hs[kMaxDim];
   for (int i = 0; i < kMaxDim; ++i) hs[i] = (i < D && layout == kInternal) ? g.hshift[i] : 0;
-  const int64_t goff = (layout == kInternal ? g.grid_off : g.ugrid_off) + (int64_t)c0 * g.gos;
+  const int64_t goff = layout == kInternal ? g.grid_off : g.ugrid_off;
+  const int cb = layout == kInternal ? g.cb : 1;
   const int inner = f.size[D - 1];
   const int outer = cells / inner;
   const int nrows = ncg * outer;
@@ -434,14 +436,14 @@ k_grid(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KBParam
     int64_t base;
     tile_storage<D>(g, f, hs, orow * inner, &base);
     base -= pos_mod(f.org[D - 1] - hs[D - 1], g.nos[D - 1]);
-    float2* dst = grid + goff + (int64_t)c * g.gos + base;
+    float2* dst = grid + goff + grid_at(g.gos, cb, c0 + c, base);
     const float* sre = acc_re + c * pstride + orow * inner;
     const float* sim = acc_im + c * pstride + orow * inner;
     for (int q = lane; q < inner; q += 32) {
       const int s = pos_mod(f.org[D - 1] + q - hs[D - 1], g.nos[D - 1]);
       const float2 v = make_float2(sre[q], sim[q]);
       if (it.split) *split_slot(so, it.split, c0 + c, orow * inner + q) = v;
-      else dst[s] = v;
+      else dst[(int64_t)s * cb] = v;
     }
   }
 }
@@ -481,7 +483,8 @@ k_reduce_split(const int4* __restrict__ split_tiles, const int* __restrict__ cou
     for (int i = 0; i < D; ++i) cells *= f.size[i];
     const int cbeg = (unit % coil_groups) * kSplitCoils;
     const int ncl = min(kSplitCoils, g.ncoil - cbeg);
-    const int64_t goff = (layout == kInternal ? g.grid_off : g.ugrid_off) + (int64_t)cbeg * g.gos;
+    const int64_t goff = layout == kInternal ? g.grid_off : g.ugrid_off;
+    const int cb = layout == kInternal ? g.cb : 1;
     for (int idx = threadIdx.x; idx < ncl * cells; idx += blockDim.x) {
       const int c = idx / cells, cell = idx - c * cells;
       const float2* src = split_slot(so, base + 1, cbeg + c, cell);
@@ -504,7 +507,7 @@ k_reduce_split(const int4* __restrict__ split_tiles, const int* __restrict__ cou
       }
       int64_t lin;
       tile_storage<D>(g, f, hs, cell, &lin);
-      grid[goff + (int64_t)c * g.gos + lin] = acc;
+      grid[goff + grid_at(g.gos, cb, cbeg + c, lin)] = acc;
     }
   }
 }
@@ -538,8 +541,9 @@ k_traj_grad(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KB
     ext[i] = i < D ? f.size[i] + kb.ntaps[i] - 1 : 1;
     hs[i] = (i < D && layout == kInternal) ? g.hshift[i] : 0;
   }
-  const int64_t goff = (layout == kInternal ? g.grid_off : g.ugrid_off) + (int64_t)c0 * g.gos;
-  load_region<D>(tile, grid, goff, g.gos, g, f.org, ext, hs, ncg, pstride);
+  const int64_t goff = layout == kInternal ? g.grid_off : g.ugrid_off;
+  const int cb = layout == kInternal ? g.cb : 1;
+  load_region<D>(tile, grid, goff, g.gos, cb, c0, g, f.org, ext, hs, ncg, pstride);
   __syncthreads();
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -767,6 +771,8 @@ int launch_interp(mrn_plan* P, const float2* grid, GridLayout layout, float2* ks
                   const float2* temporal, cudaStream_t st) {
   if (P->n_items_interp == 0) return MRN_OK;
   const bool fast = P->use_fast && fast_path_ok(P, false);
+  if (fast && !temporal && P->reg_interp && gather_ok(P, (int)layout))
+    return launch_interp_gather(P, grid, (int)layout, ksp, scale, st);
   const Layout L = plan_layout(P, 0, fast);
   const int G = pick_g(L.cg);
   dim3 gridDim((unsigned)P->n_items_interp, (unsigned)((P->max_coil + L.cg - 1) / L.cg));

@@ -83,7 +83,7 @@ __device__ __forceinline__ void sample_weights(const float* u, const int* lo, co
 // Region loader (tile + halo, wrapped), one warp per row.
 template <int D>
 __device__ __forceinline__ void load_region_f(float2* __restrict__ tile, const float2* __restrict__ grid,
-                                              int64_t goff, int64_t gos, const int* nos,
+                                              int64_t goff, int64_t gos, int cb, int c0, const int* nos,
                                               const int* org, const int* ext, const int* hs, int ncg,
                                               int pstride) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -110,12 +110,12 @@ __device__ __forceinline__ void load_region_f(float2* __restrict__ tile, const f
       base = base * nos[i] + wrap_once(org[i] + l[i] - hs[i], nos[i]);
       lbase = lbase * ext[i] + l[i];
     }
-    const float2* src = grid + goff + (int64_t)c * gos + base * nl;
+    const float2* src = grid + goff + grid_at(gos, cb, c0 + c, base * nl);
     float2* dst = tile + c * pstride + lbase * inner;
     for (int q = lane; q < inner; q += 32) {
       int s = s_first + q;
       while (s >= nl) s -= nl;
-      dst[q] = __ldg(src + s);
+      dst[q] = __ldg(src + (int64_t)s * cb);
     }
   }
 }
@@ -151,7 +151,8 @@ k_interp_fast(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, 
 #pragma unroll
   for (int i = 0; i < kMaxDim; ++i) ext[i] = i < D ? f.size[i] + K - 1 : 1;
   const int64_t gos = gp->gos;
-  const int64_t goff = (layout == kInternal ? gp->grid_off : gp->ugrid_off) + (int64_t)c0 * gos;
+  const int64_t goff = layout == kInternal ? gp->grid_off : gp->ugrid_off;
+  const int cb = layout == kInternal ? gp->cb : 1;
   const int64_t m = gp->m, pt_off = gp->pt_off, ksp_off = gp->ksp_off;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -162,7 +163,7 @@ k_interp_fast(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, 
   float4 c_next = coord[it.start + min(el, ecl)];
   int p_next = perm[it.start + min(el, ecl)];
 
-  load_region_f<D>(tile, grid, goff, gos, nos, f.org, ext, hs, ncg, pstride);
+  load_region_f<D>(tile, grid, goff, gos, cb, c0, nos, f.org, ext, hs, ncg, pstride);
   __syncthreads();
 
   for (int base = warp * SLOTS; base < it.count; base += STRIDE) {
@@ -373,7 +374,8 @@ k_grid_fast(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KB
 
   // write-back, one warp per row of the tile
   const int64_t gos = gp->gos;
-  const int64_t goff = (layout == kInternal ? gp->grid_off : gp->ugrid_off) + (int64_t)c0 * gos;
+  const int64_t goff = layout == kInternal ? gp->grid_off : gp->ugrid_off;
+  const int cb = layout == kInternal ? gp->cb : 1;
   const int inner = f.size[D - 1];
   const int outer = cells / inner;
   const int nrows = ncg * outer;
@@ -392,7 +394,7 @@ k_grid_fast(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KB
     int64_t base = 0;
 #pragma unroll
     for (int i = 0; i < D - 1; ++i) base = base * nos[i] + wrap_once(f.org[i] + l[i] - hs[i], nos[i]);
-    float2* dst = grid + goff + (int64_t)c * gos + base * nl;
+    float2* dst = grid + goff + grid_at(gos, cb, c0 + c, base * nl);
     const float* sre = acc_re + c * pstride + orow * inner;
     const float* sim = acc_im + c * pstride + orow * inner;
     for (int q = lane; q < inner; q += 32) {
@@ -400,7 +402,7 @@ k_grid_fast(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KB
       if (s >= nl) s -= nl;
       const float2 v = make_float2(sre[q], sim[q]);
       if (it.split) *split_slot(so, it.split, c0 + c, orow * inner + q) = v;
-      else dst[s] = v;
+      else dst[(int64_t)s * cb] = v;
     }
   }
 }
@@ -507,15 +509,16 @@ k_grid_warp(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KB
 
   // write-back: lanes over the cells of one coil plane at a time
   const int64_t gos = gp->gos;
-  const int64_t goff = (layout == kInternal ? gp->grid_off : gp->ugrid_off) + (int64_t)c0 * gos;
+  const int64_t goff = layout == kInternal ? gp->grid_off : gp->ugrid_off;
+  const int cb = layout == kInternal ? gp->cb : 1;
   for (int c = 0; c < ncg; ++c) {
-    float2* dstc = grid + goff + (int64_t)c * gos;
+    float2* dstc = grid + goff + grid_at(gos, cb, c0 + c, 0);
     const float2* src = acc + c * pstride;
     for (int cell = lane; cell < cells; cell += 32) {
       const int l0 = cell / size1, l1 = cell - l0 * size1;
       const int s0 = wrap_once(f.org[0] + l0 - hs0, nos0);
       const int s1 = wrap_once(f.org[1] + l1 - hs1, nos1);
-      float2* d = dstc + (int64_t)s0 * nos1 + s1;
+      float2* d = dstc + ((int64_t)s0 * nos1 + s1) * cb;
       const float2 v = src[cell];
       if (it.split) *split_slot(so, it.split, c0 + c, cell) = v;
       else *d = v;
@@ -543,7 +546,7 @@ k_grid_warp(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KB
 // 2 * CS apart (CS odd: no bank conflict).
 template <int D, int CS>
 __device__ __forceinline__ void load_region_cc(float2* __restrict__ region, const float2* __restrict__ gbase,
-                                               int64_t gos, int ncg, const Frame& f, const int* ext,
+                                               int64_t gos, int cb, int c0, int ncg, const Frame& f, const int* ext,
                                                const int* nos, const int* hs, int tid, int nthreads) {
   constexpr int kLoadBatch = 8;
   const int inner = ext[D - 1];
@@ -561,16 +564,22 @@ __device__ __forceinline__ void load_region_cc(float2* __restrict__ region, cons
              wrap_cells(f.org[1] + y - hs[1], nos[1])) * nos[2] +
             wrap_cells(f.org[2] + z - hs[2], nos[2]);
     }
-    const float2* src = gbase + off;
     float2* dst = region + cell * CS;
-    for (int cb = 0; cb < ncg; cb += kLoadBatch) {
+    const float2* src = gbase + (int64_t)c0 * gos + off;
+    for (int q0 = 0; q0 < ncg; q0 += kLoadBatch) {
       float2 v[kLoadBatch];
+      if (cb == 1) {
+#pragma unroll
+        for (int u = 0; u < kLoadBatch; ++u)
+          if (q0 + u < ncg) v[u] = __ldg(src + (int64_t)(q0 + u) * gos);
+      } else {
+#pragma unroll
+        for (int u = 0; u < kLoadBatch; ++u)
+          if (q0 + u < ncg) v[u] = __ldg(gbase + grid_at(gos, cb, c0 + q0 + u, off));
+      }
 #pragma unroll
       for (int u = 0; u < kLoadBatch; ++u)
-        if (cb + u < ncg) v[u] = __ldg(src + (int64_t)(cb + u) * gos);
-#pragma unroll
-      for (int u = 0; u < kLoadBatch; ++u)
-        if (cb + u < ncg) dst[cb + u] = v[u];
+        if (q0 + u < ncg) dst[q0 + u] = v[u];
     }
   }
 }
@@ -647,7 +656,8 @@ k_interp_reg(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, K
   }
   const int inner = ext[D - 1];
   const int64_t gos = gp->gos;
-  const float2* gbase = grid + (layout == kInternal ? gp->grid_off : gp->ugrid_off) + (int64_t)c0 * gos;
+  const float2* gbase = grid + (layout == kInternal ? gp->grid_off : gp->ugrid_off);
+  const int cb = layout == kInternal ? gp->cb : 1;
   const int64_t m = gp->m, pt_off = gp->pt_off;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int coil = lane % CW, sub = lane / CW;
@@ -661,7 +671,7 @@ k_interp_reg(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, K
       s_u[j] = coord[it.start + sb + j];
       s_p[j] = (int)(perm[it.start + sb + j] - pt_off);
     }
-    if (sb == 0) load_region_cc<D, CS>(region, gbase, gos, ncg, f, ext, nos, hs, tid, NT);
+    if (sb == 0) load_region_cc<D, CS>(region, gbase, gos, cb, c0, ncg, f, ext, nos, hs, tid, NT);
     __syncthreads();
 
     for (int base = warp * SUB; base < ns; base += NW * SUB) {
@@ -809,7 +819,8 @@ k_trajgrad_reg(const Item* __restrict__ items, const SliceGeom* __restrict__ sl,
   }
   const int inner = ext[D - 1];
   const int64_t gos = gp->gos;
-  const float2* gbase = grid + (layout == kInternal ? gp->grid_off : gp->ugrid_off) + (int64_t)c0 * gos;
+  const float2* gbase = grid + (layout == kInternal ? gp->grid_off : gp->ugrid_off);
+  const int cb = layout == kInternal ? gp->cb : 1;
   const int64_t m = gp->m, pt_off = gp->pt_off;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int coil = lane % CW, sub = lane / CW;
@@ -824,7 +835,7 @@ k_trajgrad_reg(const Item* __restrict__ items, const SliceGeom* __restrict__ sl,
       s_u[j] = coord[it.start + sb + j];
       s_p[j] = perm[it.start + sb + j];
     }
-    if (sb == 0) load_region_cc<D, CS>(region, gbase, gos, ncg, f, ext, nos, hs, tid, NT);
+    if (sb == 0) load_region_cc<D, CS>(region, gbase, gos, cb, c0, ncg, f, ext, nos, hs, tid, NT);
     __syncthreads();
 
     for (int base = warp * SUB; base < ns; base += NW * SUB) {
@@ -1123,14 +1134,15 @@ k_grid_reg(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KBP
     const int hs0 = layout == kInternal ? gp->hshift[0] : 0;
     const int hs1 = layout == kInternal ? gp->hshift[1] : 0;
     const int64_t gos = gp->gos;
-    float2* dst = grid + (layout == kInternal ? gp->grid_off : gp->ugrid_off) + (int64_t)c0 * gos +
-                  (int64_t)wrap_once(f.org[0] + row - hs0, nos0) * nos1 + wrap_once(f.org[1] + col - hs1, nos1);
+    const int cb = layout == kInternal ? gp->cb : 1;
+    float2* dst = grid + (layout == kInternal ? gp->grid_off : gp->ugrid_off);
+    const int64_t cell = (int64_t)wrap_once(f.org[0] + row - hs0, nos0) * nos1 + wrap_once(f.org[1] + col - hs1, nos1);
     const int scell = row * f.size[1] + col;
 #pragma unroll 4
     for (int c = 0; c < ncg; ++c) {
       const float2 val = sm.stage[c][tid];
       if (it.split) *split_slot(so, it.split, c0 + c, scell) = val;
-      else dst[(int64_t)c * gos] = val;
+      else dst[grid_at(gos, cb, c0 + c, cell)] = val;
     }
   }
 }

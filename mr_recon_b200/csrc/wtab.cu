@@ -150,7 +150,8 @@ k_interp_tab(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, i
   const Frame2 f = frame2(*gp, it.tile, false);
   const int ext0 = f.size[0] + ktaps.x - 1, ext1 = f.size[1] + ktaps.y - 1;
   const int64_t gos = gp->gos;
-  const int64_t goff = (layout == kInternal ? gp->grid_off : gp->ugrid_off) + (int64_t)c0 * gos;
+  const int64_t goff = layout == kInternal ? gp->grid_off : gp->ugrid_off;
+  const int cb = layout == kInternal ? gp->cb : 1;
   const int64_t m = gp->m, pt_off = gp->pt_off, ksp_off = gp->ksp_off;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slot = lane / G, lg = lane % G;
@@ -162,12 +163,12 @@ k_interp_tab(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, i
     for (int row = warp; row < nrows; row += kWarps) {
       const int c = row / ext0, l0 = row - c * ext0;
       const int sx = wrap1(f.org[0] + l0 - hs0, nos0);
-      const float2* src = grid + goff + (int64_t)c * gos + (int64_t)sx * nos1;
+      const float2* src = grid + goff + grid_at(gos, cb, c0 + c, (int64_t)sx * nos1);
       float2* dst = tile + c * pstride + l0 * ext1;
       for (int q = lane; q < ext1; q += 32) {
         int s = s_first + q;
         while (s >= nos1) s -= nos1;
-        dst[q] = __ldg(src + s);
+        dst[q] = __ldg(src + (int64_t)s * cb);
       }
     }
   }
@@ -369,15 +370,16 @@ k_grid_warp_tab(const Item* __restrict__ items, const SliceGeom* __restrict__ sl
   __syncwarp();
 
   const int64_t gos = gp->gos;
-  const int64_t goff = (layout == kInternal ? gp->grid_off : gp->ugrid_off) + (int64_t)c0 * gos;
+  const int64_t goff = layout == kInternal ? gp->grid_off : gp->ugrid_off;
+  const int cb = layout == kInternal ? gp->cb : 1;
   for (int c = 0; c < ncg; ++c) {
-    float2* dstc = grid + goff + (int64_t)c * gos;
+    float2* dstc = grid + goff + grid_at(gos, cb, c0 + c, 0);
     const float2* src = acc + c * pstride;
     for (int cell = lane; cell < cells; cell += 32) {
       const int l0 = cell / size1, l1 = cell - l0 * size1;
       const int s0 = wrap1(f.org[0] + l0 - hs0, nos0);
       const int s1 = wrap1(f.org[1] + l1 - hs1, nos1);
-      float2* d = dstc + (int64_t)s0 * nos1 + s1;
+      float2* d = dstc + ((int64_t)s0 * nos1 + s1) * cb;
       const float2 v = src[cell];
       if (it.split) *split_slot(so, it.split, c0 + c, cell) = v;
       else *d = v;

@@ -1,0 +1,88 @@
+"""The grid in coil blocks: the native FFT passes over every kind of length
+(two, three and four stages, all radices, odd image sizes) and coil counts
+around the block widths, and the interpolation kernels that read it, against
+64-bit transforms and the oracle."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import nufft_oracle as O
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _rel(a, b):
+    return float(np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+def _image_of(n):
+    """An image length whose 1.25-oversampled grid has n points, or n itself (no oversampling)."""
+    k = int(n / 1.25)
+    return (k, 1.25) if math.ceil(1.25 * k) == n else (n, 1.0)
+
+
+LENGTHS = [5, 6, 15, 16, 20, 27, 36, 50, 64, 81, 96, 100, 125, 144, 162, 200, 225, 240, 243, 250, 256, 288, 320, 375,
+           400, 432, 500, 512, 600, 625, 640, 729, 768, 810, 960, 1000, 1024]
+
+
+@pytest.mark.parametrize("n", LENGTHS)
+@pytest.mark.parametrize("last", [False, True])
+def test_native_fft_lengths(n, last):
+    from mr_recon_b200.plan import Plan
+    k, os_ = _image_of(n)
+    other = 8 if os_ > 1 else 10  # 10 grid points
+    im = (other, k) if last else (k, other)
+    C = 3
+    rng = np.random.RandomState(n + last)
+    p = Plan([im], [0], [C], os_, (4.0, 4.0), beta=9.0, device=DEV)
+    assert p.fft_kind == 1
+    nos = p.os_sizes[0]
+    img = (rng.randn(C, *im) + 1j * rng.randn(C, *im)).astype(np.complex64)
+    grid = torch.empty((C, *nos), dtype=torch.complex64, device=DEV)
+    back = torch.empty((C, *im), dtype=torch.complex64, device=DEV)
+    p.forward_ft(torch.from_numpy(img).to(DEV), grid)
+    src = (rng.randn(C, *nos) + 1j * rng.randn(C, *nos)).astype(np.complex64)
+    p.adjoint_ift(torch.from_numpy(src).to(DEV), back)
+    a = np.ones(())
+    for m, o in zip(im, nos):
+        t = np.sqrt(9.0 ** 2 - (np.pi * 4.0 * (np.arange(m) - m // 2) / o) ** 2 + 0j)
+        a = a[..., None] * (t / np.sinh(t)).real
+    a = a / math.sqrt(np.prod(im))
+    at = tuple(slice(o // 2 - m // 2, o // 2 - m // 2 + m) for m, o in zip(im, nos))
+    pad = np.zeros((C, *nos), np.complex128)
+    pad[(slice(None), *at)] = img * a
+    ax = (1, 2)
+    want = np.fft.fftshift(np.fft.fftn(np.fft.ifftshift(pad, axes=ax), axes=ax), axes=ax)
+    wback = np.fft.fftshift(np.fft.ifftn(np.fft.ifftshift(src.astype(np.complex128), axes=ax), axes=ax, norm="forward"),
+                            axes=ax)[(slice(None), *at)] * a
+    # float32 butterflies: a few ulp (6e-8) per stage, at most five stages an axis
+    assert _rel(grid.cpu().numpy(), want) < 1e-6
+    assert _rel(back.cpu().numpy(), wback) < 1e-6
+
+
+CASES = [((40, 32), 1.25, 4, 1), ((40, 32), 1.25, 6, 2), ((48, 40), 1.25, 6, 3), ((40, 32), 2.0, 5, 7), ((40, 32), 1.25, 7, 8),
+         ((48, 40), 1.25, 6, 9), ((40, 32), 1.25, 6, 17), ((40, 32), 1.5, 4, 33),
+         ((16, 12, 20), 1.25, 4, 1), ((16, 12, 20), 1.25, 6, 2), ((12, 16, 8), 2.0, 5, 4), ((16, 12, 20), 1.25, 4, 8),
+         ((12, 16, 20), 1.25, 6, 9), ((12, 8, 16), 1.25, 7, 19)]
+
+
+@pytest.mark.parametrize("im,os_,W,C", CASES)
+@pytest.mark.parametrize("M", [1, 33, 700])
+def test_interpolation_from_coil_blocks(im, os_, W, C, M):
+    """Forward over coil counts on both sides of a block, with samples on grid points, at exact kernel edges, at
+    the grid's seam and outside it."""
+    from mr_recon_b200.fourier import b200_nufft
+    d = len(im)
+    rng = np.random.RandomState(C * 1000 + M)
+    trj = ((rng.rand(1, M, d) - 0.5) * np.array(im) * 1.2).astype(np.float32)
+    trj[:, ::7] = np.round(trj[:, ::7])
+    trj[:, 1::11] = -np.array(im) / 2.0
+    img = (rng.randn(1, C, *im) + 1j * rng.randn(1, C, *im)).astype(np.complex64)
+    nf = b200_nufft(im, oversamp=os_, width=W)
+    on = O.KBNufftOracle(im, os_, W)
+    t = torch.from_numpy(trj).to(DEV)
+    # the tolerance of the repository's parity tests (float32 weights and sums)
+    assert _rel(nf.forward(torch.from_numpy(img).to(DEV), t).cpu().numpy(), on.forward(img, trj)) < 1e-5
