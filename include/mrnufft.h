@@ -109,8 +109,9 @@ int mrn_plan_fft_kind(const mrn_plan* plan);
 #define MRN_OPT_WEIGHT_TABLES 3
 /* Work decomposition (each takes effect at the next mrn_plan_set_traj):
  * MRN_OPT_INTERP_CHUNK / MRN_OPT_GRID_CHUNK: samples per interpolation work
- * item and gridding entries per gridding work item (defaults: 256 / 256 in
- * 2D, 1024 / 4096 in 3D, 1024 in 1D); MRN_OPT_INTERP_TILE / MRN_OPT_GRID_TILE:
+ * item and gridding entries per gridding work item (defaults: 256 in 2D, 1024
+ * in 3D and 1D; gridding: from the entry count, 64 to 256 in 2D, 512 to 4096
+ * in 3D, 1024 in 1D); MRN_OPT_INTERP_TILE / MRN_OPT_GRID_TILE:
  * tile edge in grid cells, every dimension (defaults: 10 / 8 in 2D, 4 / 8 in
  * 3D, 256 in 1D). */
 #define MRN_OPT_INTERP_CHUNK 4
@@ -132,15 +133,13 @@ int mrn_plan_fft_kind(const mrn_plan* plan);
  * one-slice plan given the lane count of a larger uneven plan (the lanes its
  * widest slice needs) adds every cell in the same order as that plan. */
 #define MRN_OPT_GRID_LANES 10
-/* MRN_OPT_ENTRY_MAJOR (default 1): in 2D, mrn_plan_set_traj also builds the
- * map from samples to gridding entries and a sample buffer of 8 * (largest
- * coil count) bytes per gridding entry (about 2.7x the k-space at width 6),
- * so that mrn_sense_normal keeps its samples in entry order between the
- * interpolation and the gridding (contiguous rows instead of per-coil
- * gathers; the same bits). 0 skips both; set before mrn_plan_set_traj. */
+/* MRN_OPT_ENTRY_MAJOR (default 1): mrn_sense_normal keeps its samples
+ * sample-major (the coils of a sample side by side) between the interpolation
+ * and the gridding, where both have kernels for it; the same bits. 0: sample
+ * order per coil. Set before mrn_plan_set_traj. */
 #define MRN_OPT_ENTRY_MAJOR 11
 /* MRN_OPT_NATIVE_FFT (default 1): the FFT stage as the library's own passes
- * (one per axis, Stockham in shared memory, radices 2, 3, 4, 5, 8, 16) with the apodize /
+ * (one per axis, Stockham, radices up to 20) with the apodize /
  * zero-pad folded into the first forward pass and the crop / deapodize into
  * the last adjoint pass, the zero-padded lines skipped; used when every slice
  * has the same image and grid size and every grid size is a product of 2, 3

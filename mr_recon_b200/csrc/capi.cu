@@ -114,19 +114,19 @@ int mrn_sense_normal(mrn_plan* P, const void* x, const void* mps, const float* d
   RK(check_ready(P, true));
   if (!x || !mps || !out) return MRN_ERR_ARG;
   RK(fwd_transform(P, kPreSense, (const float2*)x, (const float2*)mps, 1.0f, ST(s)));
-  if (ent_path_ok(P)) {
-    // 2D: the samples between the two stages in gridding-entry order, with the
-    // density weight applied by the interpolation (the same products, so the
-    // same bits as the sample-order path)
-    const EntIO eio{P->d_ent_of, dcf, P->max_coil, 0};
-    { StageTimer t(P, kStageInterp, ST(s)); RK(gather_ok(P, kInternal) ? launch_interp_gather(P, P->d_grid, kInternal, P->d_ksp_ent, inv_wd(P), ST(s), eio) : launch_interp_reg(P, P->d_grid, kInternal, P->d_ksp_ent, inv_wd(P), nullptr, ST(s), eio)); }
+  if (rows_path_ok(P)) {
+    // the samples stay sample-major between the two stages, with the density
+    // weight applied by the interpolation (the same products, so the same
+    // bits as the sample-order path)
+    const RowIO rio{1, 0, dcf};
     {
-      StageTimer t(P, kStageGrid, ST(s));
-      if (P->n_items_grid > 0) {
-        RK(launch_grid_reg(P, P->d_ksp_ent, nullptr, nullptr, kInternal, P->d_grid, inv_wd(P), ST(s), P->max_coil));
-        RK(launch_reduce_split(P, kInternal, P->d_grid, ST(s)));
-      }
+      StageTimer t(P, kStageInterp, ST(s));
+      RK(gather_ok(P, kInternal) ? launch_interp_gather(P, P->d_grid, kInternal, P->d_rows, inv_wd(P), ST(s), rio)
+                                 : launch_interp_reg(P, P->d_grid, kInternal, P->d_rows, inv_wd(P), nullptr, ST(s), rio));
     }
+    StageTimer t(P, kStageGrid, ST(s));
+    RK(launch_grid_rows(P, P->d_rows, nullptr, kInternal, P->d_grid, inv_wd(P), ST(s)));
+    RK(launch_reduce_split(P, kInternal, P->d_grid, ST(s)));
   } else {
     { StageTimer t(P, kStageInterp, ST(s)); RK(launch_interp(P, P->d_grid, kInternal, P->d_ksp_tmp, inv_wd(P), nullptr, ST(s))); }
     { StageTimer t(P, kStageGrid, ST(s)); RK(launch_grid(P, P->d_ksp_tmp, dcf, kInternal, P->d_grid, inv_wd(P), ST(s))); }

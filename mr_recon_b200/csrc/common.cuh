@@ -45,6 +45,8 @@ struct SliceGeom {
   float inv_sqrt_n;      // 1 / sqrt(prod(n)) (fourier.py:462, 522)
   int native_fft;        // the slice's FFT group runs the native passes (ffx.cu),
                          // which pad and crop it themselves
+  int rs;                // sample-major rows: elements per sample (coils padded to whole blocks)
+  int64_t row_off;       // complex offset of the slice's rows
   int cb;                // coils per block of the internal grid: [coil block][cell][cb] (1: coil planes)
 };
 
@@ -77,32 +79,39 @@ struct Item {
 };
 
 // Where the items of a split gridding tile (one whose entries were cut into
-// several items) put their partial tiles: slot s holds, for every coil, the
-// tile's cells in row-major order over the tile extent. A reduction pass then
-// adds the slots of each split tile in item order and stores the sum, so the
+// several items) put their partial tiles: slot s holds, for every cell of the
+// tile in row-major order, its coils side by side. A reduction pass then adds
+// the slots of each split tile in item order and stores the sum, so the
 // result does not depend on which item finishes first.
 struct SplitOut {
-  float2* part;         // [slot][coil][cell]
-  int64_t slot_stride;  // max_coil * cell_cap
-  int cell_cap;         // cells of the largest gridding tile
+  float2* part;         // [slot][cell][coil]
+  int64_t slot_stride;  // cells of the largest gridding tile * cell_stride
+  int cell_stride;      // coils of the widest slice
   int pad;
 };
 
 __device__ __forceinline__ float2* split_slot(const SplitOut& so, int split, int coil, int cell) {
-  return so.part + (int64_t)(split - 1) * so.slot_stride + (int64_t)coil * so.cell_cap + cell;
+  return so.part + (int64_t)(split - 1) * so.slot_stride + (int64_t)cell * so.cell_stride + coil;
 }
 
-// Entry-major samples of a normal operator (2D): between interpolation and
-// gridding the samples live as [gridding entry][stride] (coil c of entry e
-// at e * stride + c), so the interpolation writes one contiguous row of coils
-// per entry of the sample and the gridding reads each batch of entries as
-// one contiguous block instead of gathering one value per coil row.
-struct EntIO {
-  const int* ent_of;  // interpolation: per global point, its gridding entries, [pt][4], -1 past the last
-  const float* dcf;   // interpolation: density weight folded in before the write (or null)
-  int stride;         // > 0: entry-major samples
+// Output of an interpolation as rows (sample-major: the coils of a sample side
+// by side, SliceGeom::rs apart), the density weight of the sample applied: the
+// form the register-tile gridding reads.
+struct RowIO {
+  int on;
   int pad;
+  const float* dcf;  // or null
 };
+
+// Low bits of a gridding entry's sort key (gridrows.cu): the start z0 of its
+// window along the last axis, below NW = 10 - K <= 5, or NW where all K
+// candidate taps lie inside the tile; above it, in tiles that are cut into
+// several items, the entry's part of the trajectory, so that an item holds
+// entries of all windows (a cell's partial sums stay as short as in
+// trajectory order) and only entries of one item are ordered by window.
+constexpr int kGWinBits = 3;
+constexpr int kGPartBits = 6;
+constexpr int kGCodeBits = kGWinBits + kGPartBits;
 
 constexpr int kKBTerms = 32;  // terms of the I0 power series kept in KBParams
 
@@ -388,7 +397,7 @@ struct mrn_plan {
   int coil_group_req = 0;  // caller's coil group, 0 = choose per kernel kind
   int max_coil = 1;
   int max_chunk = 1024;   // samples per interpolation work item
-  int grid_chunk = 1024;  // entries per gridding work item
+  int grid_chunk = 0;     // entries per gridding work item, 0 = from the entry count
   int tap_max = 8;  // compile-time tap bound used (8 or 16)
   bool use_fast = true;  // use the unrolled fixed-K tile kernels where they apply
   mrn::KBParams kb{};
@@ -460,14 +469,10 @@ struct mrn_plan {
   size_t cub_tmp_bytes = 0;
   float2* d_grid = nullptr;         // internal oversampled grid (natural order, grouped)
   float2* d_ksp_tmp = nullptr;      // sample scratch for normal operators
-  // 2D normal operator in entry-major sample order (mrn_plan_set_traj): per
-  // point its gridding entries ([M][4] then [M] counters), and the samples
-  // as [entry][max_coil]
-  int* d_ent_of = nullptr;
-  float2* d_ksp_ent = nullptr;
-  int64_t cap_ent_of = 0, cap_ksp_ent = 0;
-  bool ent_ok = false;
-  bool use_ent = true;   // option: build the entry map at mrn_plan_set_traj
+  float2* d_rows = nullptr;         // sample-major rows, [n_rows], or null if they could not be allocated
+  int64_t n_rows = 0;
+  bool code_sorted = false;  // gridding entries of a tile are sorted by their last axis' window
+  bool use_ent = true;   // option: normal operators pass their samples as rows
   void* toep = nullptr;             // Toeplitz normal operator state (toeplitz.cu), or null
   unsigned* d_sync = nullptr;       // last-block counters: [0] k_cg_dir, [1] CG sums, [2] k_post
   double* d_red = nullptr;          // CG block partial sums, [n_slices][kMaxRedBlocks]

@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kGatherWarps * 32, gather_occ(D, K))
 k_interp_gather(const int* __restrict__ slices, const int* __restrict__ first_chunk, int nsl, int chunk,
                 const SliceGeom* __restrict__ sl, KBParams kb, const float4* __restrict__ coord,
                 const int* __restrict__ perm, const float2* __restrict__ grid, int layout, float2* __restrict__ ksp,
-                float scale, EntIO eio) {
+                float scale, RowIO rio) {
   constexpr int SUB = 32 / CB, WS = gather_stride(D);
   extern __shared__ __align__(16) float s_w[];                       // [chunk][WS]
   int64_t* s_cell = reinterpret_cast<int64_t*>(s_w + chunk * WS);    // first tap's cell, ~cell where it wraps
@@ -182,24 +182,20 @@ k_interp_gather(const int* __restrict__ slices, const int* __restrict__ first_ch
       const float2 a = cell < 0 ? gather_wrap<D, K, CB>(gb, ~cell, nos[0], nos[1], nos[2], w)
                                 : gather_fast<D, K - 1, CB>(gb + cell * CB, sx, sy, w);
       float2 v = make_float2(a.x * scale, a.y * scale);
-      if (eio.stride > 0) {  // entry-major: one contiguous row of coils per entry of the sample
+      if (rio.on) {
         const int p = s_p[j];
-        if (eio.dcf) {
-          const float d = eio.dcf[p];
+        if (rio.dcf) {
+          const float d = rio.dcf[p];
           v = make_float2(v.x * d, v.y * d);
         }
-        const int4 es = *reinterpret_cast<const int4*>(eio.ent_of + (int64_t)p * 4);
-        const int ee[4] = {es.x, es.y, es.z, es.w};
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (ee[q] >= 0) ksp[(int64_t)ee[q] * eio.stride + c] = v;
+        ksp[g.row_off + (p - g.pt_off) * g.rs + c] = v;
       } else if (CB == 1) {
         kspc[(int64_t)c * m + s_p[j]] = v;
       } else {
         s_o[coil * os + j] = v;
       }
     }
-    if (CB > 1 && eio.stride == 0) {
+    if (CB > 1 && !rio.on) {
       // lanes on samples: consecutive ones of a tile are mostly consecutive
       // samples of the trajectory, so a store covers runs of a coil's row
       __syncthreads();
@@ -230,7 +226,7 @@ template <int K, int NB>
 __global__ void __launch_bounds__(kTileWarps * 32, 4)
 k_interp_tile(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KBParams kb,
               const float4* __restrict__ coord, const int* __restrict__ perm, const float2* __restrict__ grid,
-              float2* __restrict__ ksp, float scale, EntIO eio) {
+              float2* __restrict__ ksp, float scale, RowIO rio) {
   constexpr int CW = 8 * NB, CS = CW + 2, SUB = 32 / CW, R = kTileRun;
   extern __shared__ __align__(16) unsigned char tsm[];
   float2* region = reinterpret_cast<float2*>(tsm);
@@ -333,24 +329,20 @@ k_interp_tile(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, 
         }
       }
       float2 v = make_float2(acc.x * scale, acc.y * scale);
-      if (eio.stride > 0) {  // entry-major: one contiguous row of coils per entry of the sample
+      if (rio.on) {
         const int pj = __shfl_sync(0xffffffffu, p, j);
         if (j < n && coil < nc) {
-          if (eio.dcf) {
-            const float d = eio.dcf[pj];
+          if (rio.dcf) {
+            const float d = rio.dcf[pj];
             v = make_float2(v.x * d, v.y * d);
           }
-          const int4 es = *reinterpret_cast<const int4*>(eio.ent_of + (int64_t)pj * 4);
-          const int ee[4] = {es.x, es.y, es.z, es.w};
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            if (ee[q] >= 0) ksp[(int64_t)ee[q] * eio.stride + c0 + coil] = v;
+          ksp[g.row_off + (pj - g.pt_off) * g.rs + c0 + coil] = v;
         }
       } else {
         s_o[warp][j][coil] = v;
       }
     }
-    if (eio.stride == 0) {
+    if (!rio.on) {
       __syncwarp();
       const int j = lane % R;
       const int pj = __shfl_sync(0xffffffffu, p, j);
@@ -417,7 +409,7 @@ static size_t tile_smem(const mrn_plan* P, int nb) {
 }
 
 int launch_interp_gather(mrn_plan* P, const float2* grid, int layout, float2* ksp, float scale, cudaStream_t st,
-                         EntIO eio) {
+                         RowIO rio) {
   const int K = P->kb.ntaps[0];
   if (P->ndim == 2 && layout == kInternal && P->gather.size() == 1 && P->gather[0].cb == 8) {
     const int nb = P->max_coil <= 8 ? 1 : 2;
@@ -431,7 +423,7 @@ int launch_interp_gather(mrn_plan* P, const float2* grid, int layout, float2* ks
     rc = set_dynamic_smem(kern, smem);                                                                      \
     if (rc == MRN_OK)                                                                                       \
       kern<<<gd, kTileWarps * 32, smem, st>>>(P->d_items_i, P->d_slices, P->kb, P->d_coord_i, P->d_perm_i, grid, \
-                                              ksp, scale, eio);                                             \
+                                              ksp, scale, rio);                                             \
   } while (0)
 #define MRN_TILE_N(KK) if (nb == 2) MRN_TILE(KK, 2); else MRN_TILE(KK, 1)
       if (K == 5) { MRN_TILE_N(5); }
@@ -450,11 +442,11 @@ int launch_interp_gather(mrn_plan* P, const float2* grid, int layout, float2* ks
     const int sub = 32 / gs.cb;
     const int warps = std::max(2, std::min(kGatherWarps, gs.chunk / sub));
     const size_t smem = (size_t)gs.chunk * (gather_stride(P->ndim) * sizeof(float) + sizeof(int64_t) + sizeof(int)) +
-                        (gs.cb > 1 && eio.stride == 0 ? (size_t)gs.cb * (gs.chunk + 1) * sizeof(float2) : 0);
+                        (gs.cb > 1 && !rio.on ? (size_t)gs.cb * (gs.chunk + 1) * sizeof(float2) : 0);
 #define MRN_GATHER(DD, KK, CC)                                                                                 \
   k_interp_gather<DD, KK, CC><<<gs.nchunks, warps * 32, smem, st>>>(sl, sl + gs.nsl, gs.nsl, gs.chunk, P->d_slices, \
                                                                  P->kb, P->d_coord_i, P->d_perm_i, grid, layout,  \
-                                                                 ksp, scale, eio)
+                                                                 ksp, scale, rio)
 #define MRN_GATHER_C(DD, KK)              \
   if (gs.cb == 8) MRN_GATHER(DD, KK, 8);  \
   else if (gs.cb == 4) MRN_GATHER(DD, KK, 4); \

@@ -32,8 +32,8 @@ inline int grid_tile_cells(const mrn_plan* P) {
 inline SplitOut split_out(const mrn_plan* P) {
   SplitOut so;
   so.part = P->d_part;
-  so.cell_cap = grid_tile_cells(P);
-  so.slot_stride = (int64_t)P->max_coil * so.cell_cap;
+  so.cell_stride = P->max_coil;
+  so.slot_stride = (int64_t)P->max_coil * grid_tile_cells(P);
   so.pad = 0;
   return so;
 }
@@ -57,23 +57,24 @@ int launch_grid_warp(mrn_plan* P, const float2* ksp, const float* dcf, const flo
                      int layout, float2* grid, float scale, cudaStream_t st);
 bool interp_reg_ok(const mrn_plan* P);
 int launch_interp_reg(mrn_plan* P, const float2* grid, int layout, float2* ksp, float scale,
-                      const float2* temporal, cudaStream_t st, EntIO eio = EntIO{nullptr, nullptr, 0, 0});
+                      const float2* temporal, cudaStream_t st, RowIO rio = RowIO{0, 0, nullptr});
 int launch_trajgrad_reg(mrn_plan* P, const float2* grid, int layout, const float2* samples, float* out,
                         float scale, cudaStream_t st);
 // Interpolation straight from a grid in coil blocks (gather.cu)
 int gather_setup(mrn_plan* P);
 bool gather_ok(const mrn_plan* P, int layout);
 int launch_interp_gather(mrn_plan* P, const float2* grid, int layout, float2* ksp, float scale, cudaStream_t st,
-                         EntIO eio = EntIO{nullptr, nullptr, 0, 0});
-bool grid_reg_ok(const mrn_plan* P);
-bool grid_reg3_ok(const mrn_plan* P);
-int launch_grid_reg3(mrn_plan* P, const float2* ksp, const float* dcf, const float2* temporal,
-                     int layout, float2* grid, float scale, cudaStream_t st);
-int launch_grid_reg(mrn_plan* P, const float2* ksp, const float* dcf, const float2* temporal,
-                    int layout, float2* grid, float scale, cudaStream_t st, int ent_stride = 0);
-// 2D normal operator with entry-major samples (EntIO): the entry map is bound
-// and the register interpolation and gridding kernels apply
-bool ent_path_ok(const mrn_plan* P);
+                         RowIO rio = RowIO{0, 0, nullptr});
+// Register-tile gridding from sample-major rows (gridrows.cu)
+bool code_sort_ok(const mrn_plan* P);
+bool grid_rows_ok(const mrn_plan* P);
+int launch_rows(mrn_plan* P, const SliceGeom* slices, int ns, const float2* ksp, const float* dcf, float2* rows,
+                cudaStream_t st);
+int launch_grid_rows(mrn_plan* P, const float2* rows, const float2* temporal, int layout, float2* grid, float scale,
+                     cudaStream_t st);
+// A normal operator can hand its samples over as rows: the register-tile
+// gridding and an interpolation that writes them apply.
+bool rows_path_ok(const mrn_plan* P);
 int launch_reduce_split(mrn_plan* P, GridLayout layout, float2* grid, cudaStream_t st);
 // 2D weight tables (wtab.cu)
 bool wtab_applicable(const mrn_plan* P);

@@ -129,6 +129,19 @@ __global__ void k_prep_points(const SliceGeom* __restrict__ sl, int ns, int ndim
   ecnt[p] = ntouch;
 }
 
+// Start of a gridding entry's window of K - 1 cells along the last axis (tile
+// `tile` of it), or 10 - K where all K candidate taps lie inside the tile: the
+// order of the register-tile gridding's entries within a tile.
+__device__ __forceinline__ int window_code(const SliceGeom& g, const KBParams& kb, float u, int tile, int i) {
+  const int K = kb.ntaps[i], KW = K - 1, n = g.nos[i], org = tile_begin(tile, n, g.gntile[i]);
+  const int size = tile_begin(tile + 1, n, g.gntile[i]) - org;
+  const int lo = (int)ceilf(__fsub_rn(u, kb.radius[i]));
+  int st = (lo < 0 ? lo + n : (lo >= n ? lo - n : lo)) - org;
+  if (st >= size) st -= n;
+  const bool last = fabsf(__fsub_rn((float)(lo + K - 1), u)) <= kb.radius[i];
+  return last && st >= 0 && st + K <= size ? 10 - K : min(max(st, 0), size - KW);
+}
+
 // Emit (tile, point) gridding entries at the scanned offsets.
 __global__ void k_emit_entries(const SliceGeom* __restrict__ sl, int ns, int ndim, KBParams kb,
                                const float4* __restrict__ coord, int64_t npts,
@@ -157,15 +170,29 @@ __global__ void k_emit_entries(const SliceGeom* __restrict__ sl, int ns, int ndi
       }
 }
 
-// Per point, the gridding entries it was emitted as (positions after the
-// tile sort); the slot order among a point's entries does not matter.
-__global__ void k_point_entries(const int* __restrict__ perm_g, int64_t ne, int* __restrict__ ent_of,
-                                int* __restrict__ cnt) {
+// Entries per tile.
+__global__ void k_tile_hist(const unsigned* __restrict__ key, int64_t n, int* __restrict__ cnt) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ne) return;
-  const int p = perm_g[e];
-  const int k = atomicAdd(cnt + p, 1);
-  if (k < 4) ent_of[(int64_t)p * 4 + k] = (int)e;
+  if (e >= n) return;
+  const unsigned k = key[e];
+  const unsigned peers = __match_any_sync(__activemask(), k);
+  if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(cnt + k, __popc(peers));
+}
+
+// Append the window code and, in tiles of more than `chunk` entries, the part
+// of the trajectory to the tile keys.
+__global__ void k_entry_codes(const SliceGeom* __restrict__ sl, int ns, int ndim, KBParams kb,
+                              const float4* __restrict__ coord, const int* __restrict__ val,
+                              const int* __restrict__ cnt, int chunk, int64_t n, unsigned* __restrict__ key) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n) return;
+  const int t = (int)key[e], p = val[e];
+  const SliceGeom& g = sl[find_slice_by_tile(sl, ns, t, 1)];
+  const int i = ndim - 1;
+  const float4 c4 = coord[p];
+  const unsigned code = (unsigned)window_code(g, kb, i == 2 ? c4.z : c4.y, (t - g.gtile_base) % g.gntile[i], i);
+  const unsigned part = cnt[t] > chunk ? (unsigned)(((int64_t)p - g.pt_off) * (1 << kGPartBits) / g.m) : 0u;
+  key[e] = (unsigned)t << kGCodeBits | part << kGWinBits | code;
 }
 
 __global__ void k_gather_coords(const float4* __restrict__ src, const int* __restrict__ perm,
@@ -174,14 +201,14 @@ __global__ void k_gather_coords(const float4* __restrict__ src, const int* __res
   if (e < n) dst[e] = src[perm[e]];
 }
 
-__global__ void k_tile_ranges(const unsigned* __restrict__ key, int64_t n, int ntiles,
+__global__ void k_tile_ranges(const unsigned* __restrict__ key, int code_bits, int64_t n, int ntiles,
                               int* __restrict__ start, int* __restrict__ end) {
   int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
-  const unsigned k = key[e];
+  const unsigned k = key[e] >> code_bits;
   if ((int)k >= ntiles) return;
-  if (e == 0 || key[e - 1] != k) start[k] = (int)e;
-  if (e == n - 1 || key[e + 1] != k) end[k] = (int)(e + 1);
+  if (e == 0 || key[e - 1] >> code_bits != k) start[k] = (int)e;
+  if (e == n - 1 || key[e + 1] >> code_bits != k) end[k] = (int)(e + 1);
 }
 
 __global__ void k_item_counts(const int* __restrict__ start, const int* __restrict__ end,
@@ -250,6 +277,20 @@ __global__ void k_gather_items(const Item* __restrict__ src, const int* __restri
 __global__ void k_total(const int* __restrict__ off, const int* __restrict__ cnt, int64_t n,
                         int* __restrict__ out) {
   if (threadIdx.x == 0 && blockIdx.x == 0) *out = n > 0 ? off[n - 1] + cnt[n - 1] : 0;
+}
+
+// Gridding entries per work item: about six items per SM in 2D and four in 3D
+// would share E evenly; fewer entries leave the densest tiles as a tail, more
+// split tiles cost partial tiles. 2D 64..256 (256^2, 32 coils, 266 k entries:
+// 64 / 128 / 192 / 256 / 512 entries 172 / 110 / 91 / 87 / 111 us; 128^2, 1
+// coil, 44 k: 28 / 33 / 39 / 42 / 65), 3D 512..4096 (192^3, 16 coils, 20.6 M:
+// 2048 / 4096 / 8192 6.1 / 5.8 / 5.7 ms; the last one's longer partial sums
+// near the k-space centre round more).
+static int default_grid_chunk(const mrn_plan* P, int64_t E) {
+  if (P->ndim == 1) return 1024;
+  const int64_t lo = P->ndim == 2 ? 64 : 512, hi = P->ndim == 2 ? 256 : 4096;
+  const int64_t share = E / ((P->ndim == 2 ? 6 : 4) * (int64_t)P->sm_count);
+  return (int)std::min(hi, std::max(lo, share / 32 * 32));
 }
 
 static inline unsigned blocks_for(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
@@ -360,7 +401,7 @@ cudaError_t upload_slices(mrn_plan* P) {
                              cudaMemcpyHostToDevice);
   if (e != cudaSuccess || !P->d_slices_kshared) return e;
   std::vector<SliceGeom> ks(P->h_slices);
-  for (auto& g : ks) g.ksp_off = 0;
+  for (auto& g : ks) g.ksp_off = g.row_off = 0;
   return cudaMemcpy(P->d_slices_kshared, ks.data(), P->nslices * sizeof(SliceGeom), cudaMemcpyHostToDevice);
 }
 
@@ -505,8 +546,7 @@ int mrn_plan_create(mrn_plan** out, int ndim, int n_slices, const int* im_size,
   // gridding tiles: 8x8 in 2D (one warp owns a tile), else the interpolation tile
   for (int i = 0; i < ndim; ++i) P->gtile[i] = (ndim >= 2 && !tile) ? 8 : P->tile[i];
   P->max_chunk = max_chunk > 0 ? max_chunk : (ndim == 2 ? 256 : 1024);
-  // one warp grids a 2D tile item alone: shorter items keep warps balanced
-  P->grid_chunk = max_chunk > 0 ? max_chunk : (ndim == 2 ? 256 : (ndim == 3 ? 4096 : 1024));
+  P->grid_chunk = max_chunk;  // 0: from the entry count, at mrn_plan_set_traj
 
   // Slices
   int64_t img = 0, ksp = 0, ugrid = 0, trjo = 0, pts = 0, xo = 0;
@@ -538,6 +578,11 @@ int mrn_plan_create(mrn_plan** out, int ndim, int n_slices, const int* im_size,
     g.ncoil = n_coil[s];
     g.m = n_pts[s];
     g.pt_off = pts;
+    // rows start on 64 bytes (one-coil plans: the samples themselves)
+    const int cbl = coil_block(g.ncoil);
+    g.rs = (g.ncoil + cbl - 1) / cbl * cbl;
+    g.row_off = maxc == 1 ? ksp : P->n_rows;
+    P->n_rows += ((int64_t)g.rs * g.m + 7) / 8 * 8;
     g.img_off = img;
     g.ksp_off = ksp;
     g.ugrid_off = ugrid;
@@ -696,6 +741,15 @@ int mrn_plan_create(mrn_plan** out, int ndim, int n_slices, const int* im_size,
     PK(cufft_setup(P));
   }
   PK(gather_setup(P));
+  if (ndim >= 2) {
+    // without room for the rows the plan grids from coil rows (the tile
+    // kernels in shared memory)
+    e = cudaMalloc((void**)&P->d_rows, std::max<int64_t>(P->n_rows, 1) * sizeof(float2));
+    if (e != cudaSuccess) {
+      P->d_rows = nullptr;
+      cudaGetLastError();
+    }
+  }
 #undef PK
   *out = P;
   return MRN_OK;
@@ -722,7 +776,7 @@ int mrn_plan_set_option(mrn_plan* P, int option, int value) {
     case MRN_OPT_REG_INTERP: P->reg_interp = value != 0; return MRN_OK;
     case MRN_OPT_ENTRY_MAJOR:
       P->use_ent = value != 0;
-      P->traj_set = false;  // the entry map is built (or not) at mrn_plan_set_traj
+      P->traj_set = false;  // takes effect at the next mrn_plan_set_traj
       return MRN_OK;
     case MRN_OPT_NATIVE_FFT:
       P->use_ffx = value != 0;
@@ -789,8 +843,7 @@ int mrn_plan_destroy(mrn_plan* P) {
                   P->d_items_g, P->d_counts, P->d_split_tiles, P->d_cub_tmp, P->d_grid,
                   P->d_ksp_tmp, P->d_sync, P->d_wmeta_i, P->d_wtab_i, P->d_wmeta_g,
                   P->d_wtab_g, P->d_part, P->d_items_tmp, P->d_sort_key[0], P->d_sort_key[1],
-                  P->d_sort_idx[0], P->d_sort_idx[1], P->d_red, P->d_rowpart, P->d_ent_of,
-                  P->d_ksp_ent, P->d_gather};
+                  P->d_sort_idx[0], P->d_sort_idx[1], P->d_red, P->d_rowpart, P->d_rows, P->d_gather};
   for (void* b : bufs)
     if (b) cudaFree(b);
   delete P;
@@ -847,7 +900,10 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
   const int ndim = P->ndim;
   int bits = 1;
   while (bits < 31 && (1ll << bits) <= (long long)TT) ++bits;
+  const int code_bits = code_sort_ok(P) && bits + kGCodeBits <= 31 ? kGCodeBits : 0;
+  const int gbits = bits + code_bits;
   P->traj_set = false;
+  P->code_sorted = code_bits > 0;
 
   // 1. coordinates, interpolation keys, gridding entry counts
   int* eoff = P->d_entry_cnt + std::max<int64_t>(M, 1);
@@ -878,6 +934,7 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
     E = hE;
   }
   P->n_entries_grid = E;
+  const int gchunk = P->grid_chunk > 0 ? P->grid_chunk : default_grid_chunk(P, E);
 
   // 2. gridding entry buffers grow on demand
   const int64_t capE = std::max<int64_t>(E, 1);
@@ -894,17 +951,23 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
   if (M > 0) {
     k_emit_entries<<<blocks_for(M), 256, 0, st>>>(P->d_slices, P->nslices, ndim, P->kb,
                                                    P->d_coord_tmp, M, eoff, P->d_key_b, P->d_val_b);
+    if (code_bits > 0 && E > 0) {
+      CK(cudaMemsetAsync(P->d_tile_end_g, 0, TG * sizeof(int), st));  // counts, until the ranges are built
+      k_tile_hist<<<blocks_for(E), 256, 0, st>>>(P->d_key_b, E, P->d_tile_end_g);
+      k_entry_codes<<<blocks_for(E), 256, 0, st>>>(P->d_slices, P->nslices, ndim, P->kb, P->d_coord_tmp, P->d_val_b,
+                                                   P->d_tile_end_g, gchunk, E, P->d_key_b);
+    }
     CK(cudaGetLastError());
     b = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, b, P->d_key_b, P->d_key_g, P->d_val_b, P->d_perm_g,
-                                    (int)std::max<int64_t>(E, 1), 0, bits, st);
+                                    (int)std::max<int64_t>(E, 1), 0, gbits, st);
     RK(ensure_cub(P, std::max(b, P->cub_tmp_bytes)));
     b = P->cub_tmp_bytes;
     CK(cub::DeviceRadixSort::SortPairs(P->d_cub_tmp, b, P->d_key_a, P->d_key_is, P->d_val_a,
                                        P->d_perm_i, (int)M, 0, bits, st));
     b = P->cub_tmp_bytes;
     CK(cub::DeviceRadixSort::SortPairs(P->d_cub_tmp, b, P->d_key_b, P->d_key_g, P->d_val_b,
-                                       P->d_perm_g, (int)E, 0, bits, st));
+                                       P->d_perm_g, (int)E, 0, gbits, st));
     k_gather_coords<<<blocks_for(M), 256, 0, st>>>(P->d_coord_tmp, P->d_perm_i, M, P->d_coord_i);
     if (E > 0)
       k_gather_coords<<<blocks_for(E), 256, 0, st>>>(P->d_coord_tmp, P->d_perm_g, E, P->d_coord_g);
@@ -918,10 +981,10 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
   CK(cudaMemsetAsync(P->d_tile_end_g, 0, TG * sizeof(int), st));
   CK(cudaMemsetAsync(P->d_counts, 0, 8 * sizeof(int), st));
   if (M > 0) {
-    k_tile_ranges<<<blocks_for(M), 256, 0, st>>>(P->d_key_is, M, T, P->d_tile_start_i,
+    k_tile_ranges<<<blocks_for(M), 256, 0, st>>>(P->d_key_is, 0, M, T, P->d_tile_start_i,
                                                  P->d_tile_end_i);
     if (E > 0)
-      k_tile_ranges<<<blocks_for(E), 256, 0, st>>>(P->d_key_g, E, TG, P->d_tile_start_g,
+      k_tile_ranges<<<blocks_for(E), 256, 0, st>>>(P->d_key_g, code_bits, E, TG, P->d_tile_start_g,
                                                    P->d_tile_end_g);
   }
 
@@ -932,7 +995,6 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
   // entries each (at most E / gchunk + 1 tiles) and ceil(c / gchunk) < 2 c / gchunk
   // items each (fewer than 2 E / gchunk slots).
   const int chunk = P->max_chunk;
-  const int gchunk = P->grid_chunk;
   const int64_t max_items_i = M > 0 ? (int64_t)T + M / chunk + 1 : 0;
   const int64_t max_items_g = (int64_t)TG + E / gchunk + 1;
   const int64_t max_split = E > gchunk ? std::min<int64_t>(TG, E / gchunk + 1) : 0;
@@ -997,24 +1059,6 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
   RK(make_items(T, chunk, 0, max_items_i, 0, 0, P->d_tile_start_i, P->d_tile_end_i, P->d_items_i));
   RK(make_items(TG, gchunk, 1, max_items_g, 1, 1, P->d_tile_start_g, P->d_tile_end_g, P->d_items_g));
   RK(build_wtabs(P, st));
-  // 2D (at most 4 entries per point): the entry map of the entry-major normal operator
-  P->ent_ok = false;
-  if (P->use_ent && ndim == 2 && !(P->flags & MRN_PLAN_RAW) && M > 0 && E > 0) {
-    if (P->cap_ent_of < 5 * M) {
-      RK(dev_alloc(&P->d_ent_of, (size_t)(5 * M)));
-      P->cap_ent_of = 5 * M;
-    }
-    const int64_t ke = E * (int64_t)P->max_coil;
-    if (P->cap_ksp_ent < ke) {
-      RK(dev_alloc(&P->d_ksp_ent, (size_t)ke));
-      P->cap_ksp_ent = ke;
-    }
-    CK(cudaMemsetAsync(P->d_ent_of, 0xff, (size_t)(4 * M) * sizeof(int), st));
-    CK(cudaMemsetAsync(P->d_ent_of + 4 * M, 0, (size_t)M * sizeof(int), st));
-    k_point_entries<<<blocks_for(E), 256, 0, st>>>(P->d_perm_g, E, P->d_ent_of, P->d_ent_of + 4 * M);
-    CK(cudaGetLastError());
-    P->ent_ok = true;
-  }
   P->n_items_interp = max_items_i;
   P->n_items_grid = max_items_g;
   P->n_split = max_split;

@@ -449,66 +449,54 @@ k_grid(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KBParam
 }
 
 // Sum the partial tiles of every split gridding tile in item order and store
-// the result. Work units are (split tile, group of kSplitCoils coils); a
-// grid of a few CTAs per SM strides over them (the number of split tiles is
-// known only on the device, counts[3]), threads over (coil, cell), each
-// thread adding the tile's slots first to last with four loads in flight.
-// The gridding kernel ran before on the same stream and wrote every slot
-// read here (a split tile's items are slots base .. base + n - 1).
-constexpr int kSplitCoils = 8;
-
+// the result. A work unit is 256 consecutive (cell, coil) values of a split
+// tile, one per thread, which adds the tile's slots first to last with 16
+// loads in flight (a unit of 512 values with 4 in flight took 39 us for the
+// 175 split tiles of 256^2, 32 coils, 98,304 spiral samples, as long as half
+// of the gridding, now 15). Blocks stride over the units (the number
+// of split tiles is known only on the device, counts[3]). The gridding kernel
+// ran before on the same stream and wrote every slot read here (a split
+// tile's items are slots base .. base + n - 1).
 template <int D>
 __global__ void __launch_bounds__(256)
 k_reduce_split(const int4* __restrict__ split_tiles, const int* __restrict__ counts,
-               const SliceGeom* __restrict__ sl, int ns, int coil_groups, SplitOut so,
+               const SliceGeom* __restrict__ sl, int ns, int units_per_tile, SplitOut so,
                float2* __restrict__ grid, int layout) {
-  const int units = counts[3] * coil_groups;
+  const int units = counts[3] * units_per_tile;
   for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
-    const int4 sp = split_tiles[unit / coil_groups];
+    const int4 sp = split_tiles[unit / units_per_tile];
     const int t = sp.x, base = sp.y, nparts = sp.z;
-    int s = 0;
-    {
-      int lo = 0, hi = ns - 1;
-      while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (sl[mid].gtile_base <= t) lo = mid; else hi = mid - 1;
-      }
-      s = lo;
+    int lo = 0, hi = ns - 1;
+    while (lo < hi) {
+      int mid = (lo + hi + 1) >> 1;
+      if (sl[mid].gtile_base <= t) lo = mid; else hi = mid - 1;
     }
-    const SliceGeom& g = sl[s];
+    const SliceGeom& g = sl[lo];
     const TileFrame f = tile_frame(g, t - g.gtile_base, D, true);
-    int hs[kMaxDim];
-    for (int i = 0; i < kMaxDim; ++i) hs[i] = (i < D && layout == kInternal) ? g.hshift[i] : 0;
     int cells = 1;
     for (int i = 0; i < D; ++i) cells *= f.size[i];
-    const int cbeg = (unit % coil_groups) * kSplitCoils;
-    const int ncl = min(kSplitCoils, g.ncoil - cbeg);
-    const int64_t goff = layout == kInternal ? g.grid_off : g.ugrid_off;
-    const int cb = layout == kInternal ? g.cb : 1;
-    for (int idx = threadIdx.x; idx < ncl * cells; idx += blockDim.x) {
-      const int c = idx / cells, cell = idx - c * cells;
-      const float2* src = split_slot(so, base + 1, cbeg + c, cell);
-      float2 acc = make_float2(0.f, 0.f);
-      int q = 0;
-      for (; q + 4 <= nparts; q += 4) {
-        float2 v[4];
+    const int idx = (unit % units_per_tile) * 256 + threadIdx.x;
+    const int cell = idx / g.ncoil, c = idx - cell * g.ncoil;  // lanes on the coils of a cell
+    if (cell >= cells) continue;
+    const float2* src = split_slot(so, base + 1, c, cell);
+    float2 acc = make_float2(0.f, 0.f);
+    for (int q = 0; q < nparts; q += 16) {
+      float2 v[16];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] = src[(int64_t)(q + k) * so.slot_stride];
+      for (int k = 0; k < 16; ++k) v[k] = q + k < nparts ? src[(int64_t)(q + k) * so.slot_stride] : make_float2(0.f, 0.f);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
+      for (int k = 0; k < 16; ++k)
+        if (q + k < nparts) {
           acc.x += v[k].x;
           acc.y += v[k].y;
         }
-      }
-      for (; q < nparts; ++q) {
-        const float2 v = src[(int64_t)q * so.slot_stride];
-        acc.x += v.x;
-        acc.y += v.y;
-      }
-      int64_t lin;
-      tile_storage<D>(g, f, hs, cell, &lin);
-      grid[goff + grid_at(g.gos, cb, cbeg + c, lin)] = acc;
     }
+    int hs[kMaxDim];
+    for (int i = 0; i < kMaxDim; ++i) hs[i] = (i < D && layout == kInternal) ? g.hshift[i] : 0;
+    int64_t lin;
+    tile_storage<D>(g, f, hs, cell, &lin);
+    grid[(layout == kInternal ? g.grid_off : g.ugrid_off) +
+         grid_at(g.gos, layout == kInternal ? g.cb : 1, c, lin)] = acc;
   }
 }
 
@@ -805,9 +793,9 @@ int launch_grid(mrn_plan* P, const float2* ksp, const float* dcf, GridLayout lay
 
 int launch_reduce_split(mrn_plan* P, GridLayout layout, float2* grid, cudaStream_t st) {
   if (P->n_split == 0) return MRN_OK;
-  const int groups = (P->max_coil + kSplitCoils - 1) / kSplitCoils;
+  const int groups = (int)((grid_tile_cells(P) * (int64_t)P->max_coil + 255) / 256);
   const int64_t units = P->n_split * groups;
-  const unsigned nb = (unsigned)std::max<int64_t>(1, std::min<int64_t>(units, 4 * (int64_t)P->sm_count));
+  const unsigned nb = (unsigned)std::max<int64_t>(1, std::min<int64_t>(units, 16 * (int64_t)P->sm_count));
   const SplitOut so = split_out(P);
   if (P->ndim == 1)
     k_reduce_split<1><<<nb, 256, 0, st>>>(P->d_split_tiles, P->d_counts, P->d_slices, P->nslices, groups, so, grid, (int)layout);
@@ -827,10 +815,17 @@ static int launch_grid_items(mrn_plan* P, const float2* ksp, const float* dcf, c
   const Layout L = plan_layout(P, 1, fast);
   const int G = pick_g(L.cg);
   dim3 gridDim((unsigned)P->n_items_grid, (unsigned)((P->max_coil + L.cg - 1) / L.cg));
-  if (fast && P->ndim == 3 && grid_reg3_ok(P))
-    return launch_grid_reg3(P, ksp, dcf, temporal, (int)layout, grid, scale, st);
-  if (fast && P->ndim == 2 && P->warp_grid && grid_reg_ok(P))
-    return launch_grid_reg(P, ksp, dcf, temporal, (int)layout, grid, scale, st);
+  if (fast && grid_rows_ok(P)) {
+    const float2* rows = ksp;
+    if (P->max_coil > 1 || dcf) {  // one coil's samples are rows already
+      // the low-rank adjoint grids one shared k-space block for all its slices
+      const int ns = P->d_slices == P->d_slices_kshared ? 1 : P->nslices;
+      const int rc = launch_rows(P, P->d_slices, ns, ksp, dcf, P->d_rows, st);
+      if (rc != MRN_OK) return rc;
+      rows = P->d_rows;
+    }
+    return launch_grid_rows(P, rows, temporal, (int)layout, grid, scale, st);
+  }
   if (fast && P->ndim == 2 && P->warp_grid && P->wtab_ok && P->use_wtab)
     return launch_grid_warp_tab(P, ksp, dcf, temporal, (int)layout, grid, scale, st);
   if (fast && P->ndim == 2 && P->warp_grid)

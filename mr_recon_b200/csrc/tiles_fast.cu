@@ -632,7 +632,7 @@ __global__ void __launch_bounds__(kRegInterpWarps * 32, (D == 3 && K > 5) ? 2 : 
 k_interp_reg(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KBParams kb,
              const float4* __restrict__ coord, const int* __restrict__ perm,
              const float2* __restrict__ grid, int layout, float2* __restrict__ ksp, float scale,
-             const float2* __restrict__ temporal, int cg, EntIO eio) {
+             const float2* __restrict__ temporal, int cg, RowIO rio) {
   constexpr int CW = 32 / SUB, CS = CW + 1, NW = kRegInterpWarps, NT = NW * 32;
   extern __shared__ float4 smem_f4[];
   float2* region = reinterpret_cast<float2*>(smem_f4);
@@ -705,18 +705,9 @@ k_interp_reg(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, K
         h = make_float2(scale * t.x, scale * t.y);
       }
       const float2 v = make_float2(acc.x * h.x - acc.y * h.y, acc.x * h.y + acc.y * h.x);
-      if (eio.stride > 0) {  // entry-major: one contiguous row of coils per entry of the sample
-        const int64_t pg = pt_off + lp;
-        float2 vv = v;
-        if (eio.dcf) {
-          const float d = eio.dcf[pg];
-          vv = make_float2(v.x * d, v.y * d);
-        }
-        const int4 es = *reinterpret_cast<const int4*>(eio.ent_of + pg * 4);
-        const int ee[4] = {es.x, es.y, es.z, es.w};
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (ee[q] >= 0) ksp[(int64_t)ee[q] * eio.stride + c0 + coil] = vv;
+      if (rio.on) {
+        const float d = rio.dcf ? rio.dcf[pt_off + lp] : 1.f;
+        ksp[gp->row_off + (int64_t)lp * gp->rs + c0 + coil] = rio.dcf ? make_float2(v.x * d, v.y * d) : v;
         continue;
       }
       float2* dst = kspc + lp;
@@ -912,242 +903,6 @@ k_trajgrad_reg(const Item* __restrict__ items, const SliceGeom* __restrict__ sl,
 }
 
 // ---------------------------------------------------------------------------
-// 2D gridding with the tile accumulator in registers. One block of two warps
-// per work item; lane = coil, warp w owns rows 4w..4w+3 of the (at most) 8x8
-// tile, so each lane keeps 4x8 complex cells in registers and every update
-// is a register FMA with a compile-time index: no shared-memory
-// read-modify-write, no atomics, float32 accumulation in a fixed order
-// (reproducible results; split tiles write partial tiles that a reduction
-// pass adds in item order).
-//
-// Entries run in batches of kRegBatch through an asynchronous pipeline
-// (cp.async), one barrier per batch. In iteration b:
-//   * the sample values (one 8-byte copy per entry and coil), densities and
-//     temporal weights of batch b+1 are copied into shared memory;
-//   * the coordinates and sample indices of batch b+3 are copied into a
-//     three-slot ring;
-//   * the 1D weights of batch b+1 are computed, already aligned to the
-//     tile's cells (zero outside the kernel support and the tile): thread
-//     (entry, dimension, half) evaluates 4 cells and stores them at once;
-//   * batch b accumulates: per entry, each of the warp's tile rows with a
-//     non-zero weight takes 8 packed two-lane FMAs per lane (fma.rn.f32x2:
-//     real and imaginary part of a cell in one instruction); the scale is
-//     folded into the row weights.
-// With at most 16 coils per group a warp runs SUB = 32 / CW entry streams of
-// CW lanes (CW = coil group rounded up to a power of two); their partial
-// tiles are summed with shuffles before the write-back.
-// ---------------------------------------------------------------------------
-constexpr int kRegTile = 8;
-constexpr int kRegRows = kRegTile / 2;  // tile rows per warp
-constexpr int kRegBatch = 16;
-constexpr int kRegStage = kRegTile * kRegTile + 1;  // cells per coil block in the write-back, padded
-
-// Shared memory of k_grid_reg: the batch pipeline's buffers, reused after the
-// last batch to stage the tile for the write-back.
-template <int CW>
-union G2Smem {
-  struct {
-    float4 c[3][kRegBatch];      // coordinate ring
-    int pm[3][kRegBatch];        // sample index ring
-    float4 wr[2][kRegBatch][2];  // per entry: row weights x scale (cells 0-7)
-    float4 wc[2][kRegBatch][4];  // per entry: column weights, each twice (cells 0-7)
-    float2 v[2][kRegBatch][CW + 1];  // per entry and coil: sample value (row padded: conflict-free copies)
-    float d[2][kRegBatch];       // per entry: density weight
-    float2 t[2][kRegBatch];      // per entry: temporal weight
-  } b;
-  float2 stage[CW][kRegStage];   // write-back: per coil, the tile's cells row-major
-};
-
-template <int K, int SUB>
-__global__ void __launch_bounds__(64, 8)
-k_grid_reg(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KBParams kb,
-           const float4* __restrict__ coord, const int* __restrict__ perm,
-           const float2* __restrict__ ksp, const float* __restrict__ dcf,
-           const float2* __restrict__ temporal, float2* __restrict__ grid, int layout, float scale,
-           int cg, SplitOut so, int ent_stride) {
-  constexpr int T = kRegTile, R = kRegRows, B = kRegBatch, CW = 32 / SUB;
-  __shared__ G2Smem<CW> sm;
-  auto& s_c = sm.b.c;
-  auto& s_pm = sm.b.pm;
-  auto& s_wr = sm.b.wr;
-  auto& s_wc = sm.b.wc;
-  auto& s_v = sm.b.v;
-  auto& s_d = sm.b.d;
-  auto& s_t = sm.b.t;
-
-  const Item it = items[blockIdx.x];
-  if (it.slice < 0) return;  // padding past the real items
-  const SliceGeom* gp = sl + it.slice;
-  const int ncoil = gp->ncoil;
-  const int c0 = blockIdx.y * cg;
-  if (c0 >= ncoil) return;
-  const int ncg = min(cg, ncoil - c0);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int coil = lane % CW, sub = lane / CW;
-  const int sid = warp * SUB + sub;  // copy stream of this thread
-  const bool has_coil = coil < ncg;
-  const int nos0 = gp->nos[0], nos1 = gp->nos[1];
-  const Frame f = frame_of(*gp, it.tile, 2, true);
-  const int64_t m = gp->m, pt_off = gp->pt_off;
-  const int nbatch = (it.count + B - 1) / B;
-  auto batch_len = [&](int bi) { return bi < nbatch ? min(B, it.count - bi * B) : 0; };
-
-  // coordinates and sample indices of batch bi into ring slot bi % 3
-  auto copy_coords = [&](int bi) {
-    const int nb = batch_len(bi), r3 = bi % 3;
-    if (tid < nb) cp_async16(&s_c[r3][tid], coord + it.start + bi * B + tid);
-    else if (tid >= 32 && tid - 32 < nb) cp_async4(&s_pm[r3][tid - 32], perm + it.start + bi * B + tid - 32);
-  };
-  // values (per entry and coil), densities and temporal weights of batch bi
-  auto copy_values = [&](int bi) {
-    const int nb = batch_len(bi), b2 = bi & 1, r3 = bi % 3;
-    if (ent_stride > 0) {  // entry-major samples: the batch's rows are contiguous
-      if (has_coil) {
-        const float2* eb = ksp + (int64_t)(it.start + bi * B) * ent_stride + c0 + coil;
-        for (int j = sid; j < nb; j += 2 * SUB) cp_async8(&s_v[b2][j][coil], eb + (int64_t)j * ent_stride);
-      }
-    } else {
-      // thread = (entry tid % B, coil phase tid / B): one warp copy reads 16
-      // entries of each of two coil rows, i.e. consecutive samples of a row
-      // (one or two 128-byte lines) rather than 32 coil rows
-      const int j = tid % B;
-      if (j < nb) {
-        const float2* src = ksp + gp->ksp_off + (int64_t)c0 * m + (s_pm[r3][j] - pt_off);
-        for (int c = tid / B; c < ncg; c += 64 / B) cp_async8(&s_v[b2][j][c], src + (int64_t)c * m);
-      }
-    }
-    if (tid < nb) {
-      if (dcf) cp_async4(&s_d[b2][tid], dcf + s_pm[r3][tid]);
-    } else if (tid >= 32 && tid - 32 < nb) {
-      if (temporal) cp_async8(&s_t[b2][tid - 32], temporal + s_pm[r3][tid - 32]);
-    }
-  };
-  // tile-aligned 1D weights of batch bi: thread = (entry, dimension, half of the cells)
-  auto weights = [&](int bi) {
-    const int j = tid >> 2, i = (tid >> 1) & 1, h = tid & 1;
-    if (j >= batch_len(bi)) return;
-    const float4 c4 = s_c[bi % 3][j];
-    const float u = i ? c4.y : c4.x;
-    const float r = i ? kb.radius[1] : kb.radius[0];
-    const float ir = i ? kb.inv_radius[1] : kb.inv_radius[0];
-    const int n = i ? nos1 : nos0;
-    const int size = i ? f.size[1] : f.size[0];
-    const int lo = (int)ceilf(__fsub_rn(u, r));
-    int st = wrap_once(lo, n) - (i ? f.org[1] : f.org[0]);
-    if (st >= size) st -= n;  // footprint wraps into this tile from the end
-    float w[4];
-#pragma unroll
-    for (int l = 0; l < 4; ++l) {
-      const int cell = 4 * h + l;
-      const int q = cell - st;
-      const float adx = fabsf(__fsub_rn((float)(lo + q), u));
-      w[l] = (q >= 0 && q < K && cell < size && adx <= r) ? kb_tap_fast(adx, ir, kb) : 0.f;
-    }
-    if (i == 0) {
-      s_wr[bi & 1][j][h] = make_float4(w[0] * scale, w[1] * scale, w[2] * scale, w[3] * scale);
-    } else {
-      s_wc[bi & 1][j][2 * h] = make_float4(w[0], w[0], w[1], w[1]);
-      s_wc[bi & 1][j][2 * h + 1] = make_float4(w[2], w[2], w[3], w[3]);
-    }
-  };
-
-  float2 acc[R][T];
-#pragma unroll
-  for (int a = 0; a < R; ++a)
-#pragma unroll
-    for (int b = 0; b < T; ++b) acc[a][b] = make_float2(0.f, 0.f);
-
-  copy_coords(0);
-  copy_coords(1);
-  cp_async_commit();
-  cp_async_wait<0>();
-  __syncthreads();
-  copy_values(0);
-  cp_async_commit();
-  copy_coords(2);
-  cp_async_commit();
-  weights(0);
-  for (int bi = 0; bi < nbatch; ++bi) {
-    cp_async_wait<1>();  // values of bi and coordinates of bi + 1 have landed (this thread's)
-    __syncthreads();     // ... everyone's; weights of bi visible; buffers of bi - 1 free
-    copy_values(bi + 1);
-    cp_async_commit();
-    copy_coords(bi + 3);
-    cp_async_commit();
-    weights(bi + 1);
-    const int b2 = bi & 1, nb = batch_len(bi);
-    for (int j = sub; j < nb; j += SUB) {
-      const float4 rw = s_wr[b2][j][warp];
-      const float wr[R] = {rw.x, rw.y, rw.z, rw.w};
-      float2 wc[T];
-#pragma unroll
-      for (int b = 0; b < T / 2; ++b) {
-        const float4 c = s_wc[b2][j][b];
-        wc[2 * b] = make_float2(c.x, c.y);
-        wc[2 * b + 1] = make_float2(c.z, c.w);
-      }
-      float2 val = s_v[b2][j][coil];
-      if (dcf) {
-        const float d = s_d[b2][j];
-        val = make_float2(val.x * d, val.y * d);
-      }
-      if (temporal) {  // times conj(t)
-        const float2 t = s_t[b2][j];
-        val = make_float2(val.x * t.x + val.y * t.y, val.y * t.x - val.x * t.y);
-      }
-#pragma unroll
-      for (int a = 0; a < R; ++a) {
-        if (SUB == 1 && wr[a] == 0.f) continue;  // uniform: one entry per warp
-        const float2 v2 = make_float2(wr[a] * val.x, wr[a] * val.y);
-#pragma unroll
-        for (int b = 0; b < T; ++b) acc[a][b] = __ffma2_rn(wc[b], v2, acc[a][b]);  // both lanes of the cell
-      }
-    }
-  }
-  cp_async_wait<0>();
-
-  if (SUB > 1) {
-#pragma unroll
-    for (int a = 0; a < R; ++a)
-#pragma unroll
-      for (int b = 0; b < T; ++b)
-#pragma unroll
-        for (int o = CW; o < 32; o <<= 1) {
-          acc[a][b].x += __shfl_xor_sync(0xffffffffu, acc[a][b].x, o);
-          acc[a][b].y += __shfl_xor_sync(0xffffffffu, acc[a][b].y, o);
-        }
-  }
-  // Write-back through shared memory: each lane stores its coil's cells as a
-  // row-major block (stride 65 cells: conflict-free 8-byte stores), then
-  // thread t stores cell t of every coil block, so one warp store covers four
-  // 64-byte rows of one coil instead of 32 coils' scattered 8-byte cells.
-  __syncthreads();  // batch buffers no longer read
-  if (has_coil && sub == 0) {
-#pragma unroll
-    for (int a = 0; a < R; ++a)
-#pragma unroll
-      for (int b = 0; b < T; ++b) sm.stage[coil][(warp * R + a) * T + b] = acc[a][b];
-  }
-  __syncthreads();
-  const int row = tid >> 3, col = tid & 7;
-  if (row < f.size[0] && col < f.size[1]) {
-    const int hs0 = layout == kInternal ? gp->hshift[0] : 0;
-    const int hs1 = layout == kInternal ? gp->hshift[1] : 0;
-    const int64_t gos = gp->gos;
-    const int cb = layout == kInternal ? gp->cb : 1;
-    float2* dst = grid + (layout == kInternal ? gp->grid_off : gp->ugrid_off);
-    const int64_t cell = (int64_t)wrap_once(f.org[0] + row - hs0, nos0) * nos1 + wrap_once(f.org[1] + col - hs1, nos1);
-    const int scell = row * f.size[1] + col;
-#pragma unroll 4
-    for (int c = 0; c < ncg; ++c) {
-      const float2 val = sm.stage[c][tid];
-      if (it.split) *split_slot(so, it.split, c0 + c, scell) = val;
-      else dst[grid_at(gos, cb, c0 + c, cell)] = val;
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
 // Launch helpers (called from tiles.cu when the fast path applies)
 // ---------------------------------------------------------------------------
 template <class Kern>
@@ -1272,7 +1027,7 @@ bool interp_reg_ok(const mrn_plan* P) {
 }
 
 int launch_interp_reg(mrn_plan* P, const float2* grid, int layout, float2* ksp, float scale,
-                      const float2* temporal, cudaStream_t st, EntIO eio) {
+                      const float2* temporal, cudaStream_t st, RowIO rio) {
   if (P->n_items_interp == 0) return MRN_OK;
   int cg, ng;
   const int sub = interp_reg_sub(P, &cg, &ng);
@@ -1287,7 +1042,7 @@ int launch_interp_reg(mrn_plan* P, const float2* grid, int layout, float2* ksp, 
     if (rc == MRN_OK)                                                                               \
       kern<<<gdim, kRegInterpWarps * 32, smem, st>>>(P->d_items_i, P->d_slices, P->kb, P->d_coord_i, \
                                                      P->d_perm_i, grid, layout, ksp, scale, temporal, cg, \
-                                                     eio);                                            \
+                                                     rio);                                            \
   } while (0)
 #define MRN_IREG_SUB(DD, KK)                     \
   if (sub == 4) MRN_IREG_LAUNCH(DD, KK, 4);      \
@@ -1344,44 +1099,9 @@ int launch_trajgrad_reg(mrn_plan* P, const float2* grid, int layout, const float
   return e == cudaSuccess ? MRN_OK : cuda_fail(e);
 }
 
-bool ent_path_ok(const mrn_plan* P) {
-  return P->ent_ok && P->ndim == 2 && P->use_fast && fast_path_ok(P, false) && interp_reg_ok(P) &&
-         fast_path_ok(P, true) && P->warp_grid && grid_reg_ok(P) && P->cap_ksp_ent >= P->n_entries_grid * P->max_coil;
-}
-
-bool grid_reg_ok(const mrn_plan* P) {
-  return P->reg_grid && P->ndim == 2 && P->tmax_gcells[0] <= kRegTile && P->tmax_gcells[1] <= kRegTile;
-}
-
-int launch_grid_reg(mrn_plan* P, const float2* ksp, const float* dcf, const float2* temporal,
-                    int layout, float2* grid, float scale, cudaStream_t st, int ent_stride) {
-  if (P->n_items_grid == 0) return MRN_OK;
-  int cg = P->coil_group_req > 0 ? std::min(P->coil_group_req, P->max_coil) : P->max_coil;
-  cg = std::max(1, std::min(cg, 32));
-  const int ng = (P->max_coil + cg - 1) / cg;
-  cg = (P->max_coil + ng - 1) / ng;
-  // entry streams per warp: 32 lanes / (coil group rounded up to 8, 16 or 32,
-  // or the lane count the plan option asks for when that is larger)
-  const int lanes = std::max(cg, P->grid_lanes);
-  const int sub = lanes <= 8 ? 4 : (lanes <= 16 ? 2 : 1);
-  const dim3 gdim((unsigned)P->n_items_grid, (unsigned)ng);
-  const int K = P->kb.ntaps[0];
-#define MRN_REG_LAUNCH(KK, SS)                                                              \
-  k_grid_reg<KK, SS><<<gdim, 64, 0, st>>>(P->d_items_g, P->d_slices, P->kb, P->d_coord_g, \
-                                          P->d_perm_g, ksp, dcf, temporal, grid, layout, scale, cg, \
-                                          split_out(P), ent_stride)
-#define MRN_REG_SUB(KK)                     \
-  if (sub == 4) MRN_REG_LAUNCH(KK, 4);      \
-  else if (sub == 2) MRN_REG_LAUNCH(KK, 2); \
-  else MRN_REG_LAUNCH(KK, 1)
-  if (K == 5) { MRN_REG_SUB(5); }
-  else if (K == 6) { MRN_REG_SUB(6); }
-  else if (K == 7) { MRN_REG_SUB(7); }
-  else { MRN_REG_SUB(8); }
-#undef MRN_REG_SUB
-#undef MRN_REG_LAUNCH
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? MRN_OK : cuda_fail(e);
+bool rows_path_ok(const mrn_plan* P) {
+  return P->use_ent && P->reg_interp && fast_path_ok(P, false) && fast_path_ok(P, true) && grid_rows_ok(P) &&
+         (gather_ok(P, kInternal) || interp_reg_ok(P));
 }
 
 int launch_grid_fast(mrn_plan* P, const float2* ksp, const float* dcf, const float2* temporal,

@@ -58,11 +58,11 @@ __device__ __forceinline__ void dim_table(float u, float r, float inv_r, const K
 }
 
 __global__ void k_wtab(const SliceGeom* __restrict__ sl, int ns, KBParams kb,
-                       const float4* __restrict__ coord, const unsigned* __restrict__ key, int64_t n,
-                       int gridding, int4* __restrict__ meta, float4* __restrict__ tab) {
+                       const float4* __restrict__ coord, const unsigned* __restrict__ key, int code_bits,
+                       int64_t n, int gridding, int4* __restrict__ meta, float4* __restrict__ tab) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
-  const int t = (int)key[e];
+  const int t = (int)(key[e] >> code_bits);
   const int s = slice_of_tile(sl, ns, t, gridding != 0);
   const SliceGeom& g = sl[s];
   int tile = t - (gridding ? g.gtile_base : g.tile_base);
@@ -425,10 +425,10 @@ int build_wtabs(mrn_plan* P, cudaStream_t st) {
   if (rc != MRN_OK) return rc;
   if (M > 0)
     k_wtab<<<(unsigned)((M + 255) / 256), 256, 0, st>>>(P->d_slices, P->nslices, P->kb, P->d_coord_i,
-                                                         P->d_key_is, M, 0, P->d_wmeta_i, P->d_wtab_i);
+                                                         P->d_key_is, 0, M, 0, P->d_wmeta_i, P->d_wtab_i);
   if (E > 0)
     k_wtab<<<(unsigned)((E + 255) / 256), 256, 0, st>>>(P->d_slices, P->nslices, P->kb, P->d_coord_g,
-                                                         P->d_key_g, E, 1, P->d_wmeta_g, P->d_wtab_g);
+                                                         P->d_key_g, P->code_sorted ? kGCodeBits : 0, E, 1, P->d_wmeta_g, P->d_wtab_g);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e);
   P->wtab_ok = true;

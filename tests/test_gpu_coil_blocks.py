@@ -86,3 +86,41 @@ def test_interpolation_from_coil_blocks(im, os_, W, C, M):
     t = torch.from_numpy(trj).to(DEV)
     # the tolerance of the repository's parity tests (float32 weights and sums)
     assert _rel(nf.forward(torch.from_numpy(img).to(DEV), t).cpu().numpy(), on.forward(img, trj)) < 1e-5
+
+
+GRID_CASES = [((40, 32), 1.25, 4, 1), ((40, 32), 1.25, 6, 3), ((40, 32), 2.0, 5, 6), ((40, 32), 1.25, 7, 8),
+              ((48, 40), 1.25, 6, 11), ((40, 32), 1.25, 6, 17), ((40, 32), 1.5, 4, 35),
+              ((16, 12, 20), 1.25, 4, 1), ((16, 20, 12), 1.5, 6, 3), ((12, 16, 16), 2.0, 5, 7), ((16, 16, 16), 1.5, 7, 12),
+              ((16, 12, 20), 1.25, 4, 19)]
+
+
+@pytest.mark.parametrize("im,os_,W,C", GRID_CASES)
+@pytest.mark.parametrize("chunk", [1, 40, 100000])
+def test_register_tile_gridding(im, os_, W, C, chunk):
+    """Gridding over coil counts on both sides of its lane groups, with a dense centre (split tiles, several
+    trajectory parts and windows per batch of entries), grid points and exact kernel edges, and the seam; and the
+    density-weighted normal operator, which passes rows, against the adjoint of the forward."""
+    from mr_recon_b200 import _lib
+    from mr_recon_b200.linops import sense_linop
+    from mr_recon_b200.fourier import b200_nufft
+    d, M = len(im), 500
+    rng = np.random.RandomState(C * 100 + W)
+    trj = ((rng.rand(M, d) - 0.5) * np.array(im) * 1.1).astype(np.float32)
+    trj[::2] *= 0.15
+    trj[::9] = np.round(trj[::9])
+    ksp = (rng.randn(C, M) + 1j * rng.randn(C, M)).astype(np.complex64)
+    nf = b200_nufft(im, oversamp=os_, width=W)
+    on = O.KBNufftOracle(im, os_, W)
+    t = torch.from_numpy(trj).to(DEV)
+    mps = torch.from_numpy((rng.randn(C, *im) + 1j * rng.randn(C, *im)).astype(np.complex64)).to(DEV)
+    dcf = torch.from_numpy((0.5 + rng.rand(M)).astype(np.float32)).to(DEV)
+    A = sense_linop(t, mps, dcf=dcf, nufft=nf)
+    A.plan.set_option(_lib.MRN_OPT_GRID_CHUNK, chunk)
+    A.plan.set_traj(t.reshape(-1))
+    assert (A.plan.stats()["split_tiles"] > 0) == (chunk < 500)
+    g = torch.empty((C, *A.plan.os_sizes[0]), dtype=torch.complex64, device=DEV)
+    A.plan.grid(torch.from_numpy(ksp).to(DEV), g, 1.0 / W ** d)
+    # the tolerance of the repository's parity tests (float32 weights and sums)
+    assert _rel(g.cpu().numpy(), on.adjoint_grid_only(ksp[None], trj[None])[0]) < 1e-5
+    x = torch.from_numpy((rng.randn(*im) + 1j * rng.randn(*im)).astype(np.complex64)).to(DEV)
+    assert torch.equal(A.normal(x), A.adjoint(A.forward(x)))
