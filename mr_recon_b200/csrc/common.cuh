@@ -115,49 +115,90 @@ constexpr int kGCodeBits = kGWinBits + kGPartBits;
 
 constexpr int kKBTerms = 32;  // terms of the I0 power series kept in KBParams
 
-// One axis of the native FFT (ffx.cu): length n = radix[0] * ... *
-// radix[ns - 1], at least two stages (the last may be 1), each radix at most 20; stage s reads its twiddles
-// exp(-2 pi i t j / (L R)), j < L = radix[0] * ... * radix[s - 1], 1 <= t < R,
-// at tw + tw_off[s] + j (R - 1) + t - 1 of the axis' table (n - 1 entries).
+// One axis of the native FFT. m = 0: length n = radix[0] * ... *
+// radix[ns - 1], at least two stages (the last may be 1), each radix at most
+// 20 (ffx.cu); stage s reads its twiddles exp(-2 pi i t j / (L R)), j < L =
+// radix[0] * ... * radix[s - 1], 1 <= t < R, at tw + tw_off[s] + j (R - 1) +
+// t - 1 of the axis' table. m > 0: a chirp convolution of length m =
+// radix[0] * radix[1], at least 2 n - 1 (ffxconv.cu), whose table is the m-th
+// roots of unity.
 constexpr int kFfxMaxStages = 4;
 constexpr int kFfxMaxN = 1024;
+// Lengths with a prime factor above 5 run natively from here on. Shorter grids
+// are launch-bound either way and keep cuFFT (78^2 image, 98^2 grid, 8 coils:
+// FFT stage with pad and crop 50 us natively, 49 with cuFFT; 97 x 109, 4 coils:
+// 47 and 63; 203^2, 32 coils: 151 and 298).
+constexpr int kFfxConvMin = 96;
 struct FfxAxis {
   int n;
+  int m;
   int ns;
   int radix[kFfxMaxStages];
   int tw_off[kFfxMaxStages];
   unsigned mag_l[kFfxMaxStages];   // floor(2^32 / L) + 1: b / L = umulhi(b, mag_l) for b < 2^16
-  unsigned mag_nr[kFfxMaxStages];  // the same for n / radix
-  int tw_base;  // first entry of this axis in the plan's twiddle table
+  unsigned mag_nr[kFfxMaxStages];  // the same for the butterflies of the stage
+  int tw_base;  // first entry of this axis in the twiddle table
+  int chirp;    // m > 0: its chirp (n entries) and filter (m entries) there
+  int filter;
 };
 
-// One FFT group of a grid buffer (slices of one grid size, back to back as
-// [batch][nos...]). native: its slices have the same image size and every
-// axis is a product of 2, 3 and 5 with at most kFfxMaxN points.
+// Geometry of one pass (one axis of the slices of one grid and image size).
+struct FfxPass {
+  FfxAxis ax;
+  int axis;
+  int n_img;        // image points along the axis
+  int en1, enos1;   // image and grid size of the second axis when it precedes this one, else 1
+  int pcols;        // image points of the earlier axes
+  int icells;       // grid cells of the later axes
+  int narrow;       // last axis with fewer than 8 coils per cell: adjacent columns are other lines
+};
+
+struct FfxSlice {
+  int slice, pass;  // pass: index into FfxSet::d_pass
+};
+
+// One launch of a transform: the slices whose axis `axis` runs as direct
+// radices, or as a chirp convolution.
+struct FfxStep {
+  int axis;
+  bool conv;
+  int first, nsl;     // slices at FfxSet::d_list + first
+  FfxPass pass;       // the pass, if all of them share one
+  bool one_pass;
+  int64_t max_cols;   // columns of the widest slice
+  int w, threads;     // columns per CTA, threads
+  bool big;           // direct: radices 7 to 19; chirp: radices above 20 among the passes
+  size_t smem;
+};
+
+// One FFT group of a grid buffer (slices of one grid size). native: its slices
+// have the same image size and every axis has a plan (ffx_axis).
 struct FfxGroup {
   bool native;
   FfxAxis ax[kMaxDim];
   int first_slice;  // geometry (image and grid size) shared by the group's slices
-  int nsl;          // slices in the group
-  int sl_off;       // their ids at FfxSet::d_sl + sl_off, in grid order
-  int max_coil;     // coils of the widest slice, padded to whole coil blocks
-  int total_coil;   // padded coils of all slices
 };
 
-// The native FFT of one grid buffer: its groups, their twiddle tables and
-// slice lists (host side owns the device arrays; release() frees them).
+// The native FFT of one grid buffer: its groups, the launches of each axis,
+// twiddle tables and slice lists (host side owns the device arrays; release()
+// frees them).
 struct FfxSet {
   bool ok = false;   // some group is native
   bool all = false;  // every group is native
   std::vector<FfxGroup> grp;
+  std::vector<FfxStep> step[kMaxDim];
   float2* d_tw = nullptr;
-  int* d_sl = nullptr;
+  FfxSlice* d_list = nullptr;
+  FfxPass* d_pass = nullptr;
   void release() {
     if (d_tw) cudaFree(d_tw);
-    if (d_sl) cudaFree(d_sl);
+    if (d_list) cudaFree(d_list);
+    if (d_pass) cudaFree(d_pass);
     d_tw = nullptr;
-    d_sl = nullptr;
+    d_list = nullptr;
+    d_pass = nullptr;
     grp.clear();
+    for (auto& s : step) s.clear();
     ok = all = false;
   }
 };
@@ -489,6 +530,7 @@ struct mrn_plan {
   // selects it (default) or cuFFT for every group.
   mrn::FfxSet ffx;
   bool use_ffx = true;
+  bool use_conv = false;  // axes without direct radices may run as chirp convolutions
   // Interpolation from the grid in coil blocks (gather.cu): the slices of
   // each block width, cut into CTAs of `chunk` sorted samples.
   struct GatherSet {

@@ -127,8 +127,18 @@ struct FfxGrid {
   float2* grid;
   int sm_count;
 };
-bool ffx_can(int ndim, const int* nos);  // every axis of the grid size can run natively
-int ffx_build(FfxSet& S, int ndim, const std::vector<SliceGeom>& hsl, const std::vector<FfxGroupSpec>& spec);
+bool ffx_can(int ndim, const int* nos, bool conv);  // every axis of the grid size can run natively
+int ffx_build(FfxSet& S, int ndim, const std::vector<SliceGeom>& hsl, const std::vector<FfxGroupSpec>& spec,
+              bool conv, int sm_count);
+// Direct passes with radices 7, 11, 13, 14, 17, 19 (ffxprime.cu).
+int launch_ffx_primes(const FfxSet& S, const FfxGrid& G, const FfxStep& step, bool inv, int source, bool to_image,
+                      const float2* src, const float2* mps, float2* out, float scale, cudaStream_t st);
+// Chirp-convolution passes (ffxconv.cu).
+bool ffx_conv_axis(int n, FfxAxis& ax);
+void ffx_conv_tables(FfxAxis& ax, std::vector<float2>& tab);
+void ffx_conv_shape(FfxStep& st, const std::vector<FfxPass>& passes, int64_t total_cols, int sm_count);
+int launch_ffx_conv(const FfxSet& S, const FfxGrid& G, const FfxStep& step, bool inv, int source, bool to_image,
+                    const float2* src, const float2* mps, float2* out, float scale, cudaStream_t st);
 int ffx_fwd(const FfxSet& S, const FfxGrid& G, PreMode mode, const float2* src, const float2* mps, float scale,
             cudaStream_t st);
 int ffx_inv(const FfxSet& S, const FfxGrid& G, float2* out, float scale, cudaStream_t st);

@@ -654,12 +654,20 @@ int mrn_plan_create(mrn_plan** out, int ndim, int n_slices, const int* im_size,
       }
       group_of[s] = found;
     }
+    // Chirp convolutions pay where cuFFT would stream the grid from HBM several
+    // times or run grid sizes one after the other: from a million points, or
+    // for several sizes (one 272 x 326 grid of 7 coils, 0.6 M: forward + adjoint
+    // 92 us with them, 87 with cuFFT; 254^2, 32 coils, 2.1 M: FFT stage 149
+    // and 298; 142 x 195 x 152, 6 coils, 25 M: 1.28 ms and 2.24)
+    int64_t points = 0;
+    for (const SliceGeom& g : P->h_slices) points += (int64_t)g.ncoil * g.gos;
+    P->use_conv = P->fft.size() > 1 || points >= 1000000;
     // grids that can run the native passes hold whole coil blocks; with
     // MRN_OPT_NATIVE_FFT 0 their unused coils are transformed along
     int64_t off = 0;
     for (size_t q = 0; q < P->fft.size(); ++q) {
       P->fft[q].grid_off = off;
-      const bool can = ffx_can(ndim, P->fft[q].nos);
+      const bool can = ffx_can(ndim, P->fft[q].nos, P->use_conv);
       for (int s = 0; s < n_slices; ++s)
         if (group_of[s] == (int)q) {
           SliceGeom& g = P->h_slices[s];

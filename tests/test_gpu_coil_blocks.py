@@ -24,7 +24,9 @@ def _image_of(n):
     return (k, 1.25) if math.ceil(1.25 * k) == n else (n, 1.0)
 
 
-LENGTHS = [5, 6, 15, 16, 20, 27, 36, 50, 64, 81, 96, 100, 125, 144, 162, 200, 225, 240, 243, 250, 256, 288, 320, 375,
+LENGTHS = [98, 112, 121, 143, 169, 187, 209, 247, 289, 304, 361, 374, 539, 616, 1001,  # 7, 11, 13, 17, 19
+           97, 111, 163, 206, 254, 326, 401, 466, 509,  # chirp convolutions
+           5, 6, 15, 16, 20, 27, 36, 50, 64, 81, 96, 100, 125, 144, 162, 200, 225, 240, 243, 250, 256, 288, 320, 375,
            400, 432, 500, 512, 600, 625, 640, 729, 768, 810, 960, 1000, 1024]
 
 
@@ -37,15 +39,21 @@ def test_native_fft_lengths(n, last):
     im = (other, k) if last else (k, other)
     C = 3
     rng = np.random.RandomState(n + last)
-    p = Plan([im], [0], [C], os_, (4.0, 4.0), beta=9.0, device=DEV)
+    # a second slice of another grid size: lengths without direct radices then run as chirp convolutions
+    p = Plan([im, (20, 16)], [0, 0], [C, 1], os_, (4.0, 4.0), beta=9.0, device=DEV)
     assert p.fft_kind == 1
     nos = p.os_sizes[0]
     img = (rng.randn(C, *im) + 1j * rng.randn(C, *im)).astype(np.complex64)
-    grid = torch.empty((C, *nos), dtype=torch.complex64, device=DEV)
-    back = torch.empty((C, *im), dtype=torch.complex64, device=DEV)
-    p.forward_ft(torch.from_numpy(img).to(DEV), grid)
+    both = torch.zeros(p.n_img, dtype=torch.complex64, device=DEV)
+    both[:img.size] = torch.from_numpy(img).reshape(-1).to(DEV)
+    grid = torch.empty(p.n_grid, dtype=torch.complex64, device=DEV)
+    back = torch.empty(p.n_img, dtype=torch.complex64, device=DEV)
+    p.forward_ft(both, grid)
     src = (rng.randn(C, *nos) + 1j * rng.randn(C, *nos)).astype(np.complex64)
-    p.adjoint_ift(torch.from_numpy(src).to(DEV), back)
+    gsrc = torch.zeros_like(grid)
+    gsrc[:src.size] = torch.from_numpy(src).reshape(-1).to(DEV)
+    p.adjoint_ift(gsrc, back)
+    grid, back = grid[:src.size].reshape(src.shape), back[:img.size].reshape(img.shape)
     a = np.ones(())
     for m, o in zip(im, nos):
         t = np.sqrt(9.0 ** 2 - (np.pi * 4.0 * (np.arange(m) - m // 2) / o) ** 2 + 0j)
