@@ -984,10 +984,10 @@ def main():
         if "c5" in want:
             extra["c5"] = bench_c5(dev)
 
-    # own kernels per fwd+adj step: interpolation and gridding, plus either the
+    # own kernels per fwd+adj step: interpolation, row transpose and gridding, plus either the
     # four native FFT passes (pad and crop fused) or k_pre / k_post around cuFFT,
     # plus the split-tile reduction
-    launches_per_step = 2 + (4 if stats["fft_kind"] == 1 else 2) + (1 if stats["split_tiles"] > 0 else 0)
+    launches_per_step = 3 + (4 if stats["fft_kind"] == 1 else 2) + (1 if stats["split_tiles"] > 0 else 0)
     if rank == 0:
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,

@@ -118,9 +118,9 @@ int mrn_plan_fft_kind(const mrn_plan* plan);
 #define MRN_OPT_GRID_CHUNK 5
 #define MRN_OPT_INTERP_TILE 6
 #define MRN_OPT_GRID_TILE 7
-/* MRN_OPT_REG_GRIDDING (default 1): 2D gridding tiles of at most 8x8 cells
- * keep their accumulator in registers (two warps per tile, lane = coil);
- * 0 keeps it in shared memory. Each gives the same bits from run to run. */
+/* MRN_OPT_REG_GRIDDING (default 1): 2D and 3D gridding tiles of 8 cells an
+ * axis keep their accumulators in registers (sample-major rows); 0 keeps them
+ * in shared memory. Each gives the same bits from run to run. */
 #define MRN_OPT_REG_GRIDDING 8
 /* MRN_OPT_REG_INTERP (default 1): 2D and 3D interpolation with one lane per
  * coil over the tile region staged as [cell][coil] (packed two-lane FMAs); 0
@@ -141,9 +141,12 @@ int mrn_plan_fft_kind(const mrn_plan* plan);
 /* MRN_OPT_NATIVE_FFT (default 1): the FFT stage as the library's own passes
  * (one per axis, Stockham, radices up to 20) with the apodize /
  * zero-pad folded into the first forward pass and the crop / deapodize into
- * the last adjoint pass, the zero-padded lines skipped; used when every slice
- * has the same image and grid size and every grid size is a product of 2, 3
- * and 5 of at most 1024. 0 (or any other plan) uses cuFFT between separate
+ * the last adjoint pass, the zero-padded lines skipped; 2D and 3D groups of
+ * one image and grid size whose lengths are products of 2, 3 and 5 of at most
+ * 1024, from 96 points also with factors 7 to 19, and (chirp convolution, plans
+ * of several grid sizes or large grids) any other length to 512. The Toeplitz
+ * grids follow the value at the time the kernels are set (direct lengths only).
+ * 0 (or any other plan) uses cuFFT between separate
  * pad and crop kernels. The two agree to float32 rounding, not bitwise. */
 #define MRN_OPT_NATIVE_FFT 12
 int mrn_plan_set_option(mrn_plan* plan, int option, int value);

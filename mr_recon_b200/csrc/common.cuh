@@ -203,6 +203,31 @@ struct FfxSet {
   }
 };
 
+// The turning pass of one slice: the first axis forward (radices of the plain
+// passes) and back (the same radices, last first).
+struct FfxTurn {
+  FfxAxis fwd, inv;
+  int n_img;         // image points along the axis
+  int icells;        // grid cells of the later axes
+  int buf;           // elements of a column's shared buffer
+  int pad;
+  int64_t kern_off;  // the slice's kernel
+};
+
+struct FfxTurnSet {
+  FfxTurn* d_turn = nullptr;  // per slice
+  float2* d_tw = nullptr;
+  int nsl = 0, w = 0, threads = 0;
+  bool primes = false;
+  int64_t max_cols = 0;
+  size_t smem = 0;
+  void release() {
+    if (d_turn) cudaFree(d_turn);
+    if (d_tw) cudaFree(d_tw);
+    *this = FfxTurnSet();
+  }
+};
+
 struct KBParams {
   float radius[kMaxDim];  // W_i / 2
   float beta;             // beta of dimension 0 (all dimensions when uniform_beta)

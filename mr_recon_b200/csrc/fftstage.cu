@@ -340,26 +340,34 @@ k_post_sense(const SliceGeom* __restrict__ sl, int ns, const float* __restrict__
   if (threadIdx.x == 0) *counter = 0u;
 }
 
+int launch_post_sense(mrn_plan* P, const SliceGeom* dsl, const float* apod, const float2* grid, const float2* mps,
+                      float2* out, float scale, const float2* xin, float lam, double* pap, int pap_stride,
+                      unsigned* counter, cudaStream_t st) {
+  if (P->n_xrow <= 0) return MRN_OK;
+  int nl = 1;
+  for (const auto& g : P->h_slices) nl = std::max(nl, g.n[P->ndim - 1]);
+  const unsigned threads = nl <= 64 ? 64 : (nl <= 128 ? 128 : 256);
+  const unsigned rows = (unsigned)P->n_xrow;
+  const int ns = P->nslices;
+  if (P->ndim == 1)
+    k_post_sense<1><<<rows, threads, 0, st>>>(dsl, ns, apod, grid, mps, scale, out, xin, lam, pap, pap_stride, P->d_rowpart, counter);
+  else if (P->ndim == 2)
+    k_post_sense<2><<<rows, threads, 0, st>>>(dsl, ns, apod, grid, mps, scale, out, xin, lam, pap, pap_stride, P->d_rowpart, counter);
+  else
+    k_post_sense<3><<<rows, threads, 0, st>>>(dsl, ns, apod, grid, mps, scale, out, xin, lam, pap, pap_stride, P->d_rowpart, counter);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? MRN_OK : cuda_fail(e);
+}
+
 int launch_post(mrn_plan* P, PostMode mode, const float2* mps, float2* out, float scale,
                 const float2* xin, float lam, double* pap, int pap_stride, cudaStream_t st) {
-  const int64_t nrows = mode == kPostSense ? P->n_xrow : P->n_irow;
-  if (mode != kPostSense) pap = nullptr;  // Re<x, out> exists only for the SENSE form
+  if (mode == kPostSense)
+    return launch_post_sense(P, P->d_slices, P->d_apod, P->d_grid, mps, out, scale, xin, lam, pap, pap_stride,
+                             P->d_sync + 2, st);
+  pap = nullptr;  // Re<x, out> exists only for the SENSE form
+  const int64_t nrows = P->n_irow;
   const unsigned blocks = (unsigned)((nrows + 7) / 8);
   if (blocks == 0) return MRN_OK;
-  if (mode == kPostSense) {
-    int nl = 1;
-    for (const auto& g : P->h_slices) nl = std::max(nl, g.n[P->ndim - 1]);
-    const unsigned threads = nl <= 64 ? 64 : (nl <= 128 ? 128 : 256);
-    const unsigned rows = (unsigned)nrows;
-    if (P->ndim == 1)
-      k_post_sense<1><<<rows, threads, 0, st>>>(P->d_slices, P->nslices, P->d_apod, P->d_grid, mps, scale, out, xin, lam, pap, pap_stride, P->d_rowpart, P->d_sync + 2);
-    else if (P->ndim == 2)
-      k_post_sense<2><<<rows, threads, 0, st>>>(P->d_slices, P->nslices, P->d_apod, P->d_grid, mps, scale, out, xin, lam, pap, pap_stride, P->d_rowpart, P->d_sync + 2);
-    else
-      k_post_sense<3><<<rows, threads, 0, st>>>(P->d_slices, P->nslices, P->d_apod, P->d_grid, mps, scale, out, xin, lam, pap, pap_stride, P->d_rowpart, P->d_sync + 2);
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? MRN_OK : cuda_fail(e);
-  }
   if (P->ndim == 1)
     k_post<1><<<blocks, 256, 0, st>>>(P->d_slices, P->nslices, P->d_apod, P->d_grid, mps, mode, scale, out, xin, lam, pap, pap_stride, nrows, P->d_rowpart, P->d_sync + 2);
   else if (P->ndim == 2)

@@ -123,16 +123,10 @@ int upload(T** dst, const std::vector<T>& v) {
 // Radices with a prime factor above 5: kernels of their own, whose butterflies
 // need more registers (in one kernel with the others they took the 2D passes
 // of 256^2, 32 coils from 83 to 107 us).
-bool has_primes(const FfxAxis& ax) {
-  for (int s = 0; s < ax.ns; ++s)
-    for (int f : {7, 11, 13, 17, 19})
-      if (ax.radix[s] % f == 0) return true;
-  return false;
-}
+bool has_primes(const FfxAxis& ax) { return ffx_has_primes(ax); }
 
 size_t pass_smem(const FfxAxis& ax, int w) {
-  const int r0s = ax.radix[0] + ((ax.ns == 2 && !(ax.radix[0] & 1)) ? 1 : 0);
-  const size_t a = (size_t)(ax.n / ax.radix[0]) * r0s * (w + 1);
+  const size_t a = (size_t)(ax.n / ax.radix[0]) * ffx_block_rows(ax.radix[0]) * (w + 1);
   const size_t b = ax.ns > 2 ? (size_t)ax.n * (w + 1) : 0;
   return ((size_t)ax.n + a + b) * sizeof(float2);
 }
@@ -178,6 +172,32 @@ FfxGrid plan_grid(mrn_plan* P) {
 }
 
 }  // namespace
+
+bool ffx_has_primes(const FfxAxis& ax) {
+  for (int s = 0; s < ax.ns; ++s)
+    for (int f : {7, 11, 13, 17, 19})
+      if (ax.radix[s] % f == 0) return true;
+  return false;
+}
+
+// Twiddles of a direct length (n - 1 entries appended to tab) and the index
+// constants of its stages, for the radices' order.
+void ffx_stage_tables(FfxAxis& ax, std::vector<float2>& tab) {
+  int L = 1, off = 0;
+  for (int st = 0; st < ax.ns; ++st) {
+    const int R = ax.radix[st], nr = ax.n / R;
+    ax.tw_off[st] = off;
+    ax.mag_l[st] = L > 1 ? (unsigned)((1ull << 32) / (unsigned long long)L + 1ull) : 0u;
+    ax.mag_nr[st] = nr > 1 ? (unsigned)((1ull << 32) / (unsigned long long)nr + 1ull) : 0u;
+    for (int j = 0; j < L; ++j)
+      for (int t = 1; t < R; ++t) {
+        const double ang = -2.0 * M_PI * (double)t * (double)j / (double)(L * R);
+        tab.push_back(make_float2((float)std::cos(ang), (float)std::sin(ang)));
+      }
+    off += L * (R - 1);
+    L *= R;
+  }
+}
 
 // Whether every axis of a grid can run the native passes.
 bool ffx_can(int ndim, const int* nos, bool conv) {
@@ -235,20 +255,7 @@ int ffx_build(FfxSet& S, int ndim, const std::vector<SliceGeom>& hsl, const std:
         ffx_conv_tables(ax, tab);
         continue;
       }
-      int L = 1, off = 0;
-      for (int st = 0; st < ax.ns; ++st) {
-        const int R = ax.radix[st], nr = ax.n / R;
-        ax.tw_off[st] = off;
-        ax.mag_l[st] = L > 1 ? (unsigned)((1ull << 32) / (unsigned long long)L + 1ull) : 0u;
-        ax.mag_nr[st] = nr > 1 ? (unsigned)((1ull << 32) / (unsigned long long)nr + 1ull) : 0u;
-        for (int j = 0; j < L; ++j)
-          for (int t = 1; t < R; ++t) {
-            const double ang = -2.0 * M_PI * (double)t * (double)j / (double)(L * R);
-            tab.push_back(make_float2((float)std::cos(ang), (float)std::sin(ang)));
-          }
-        off += L * (R - 1);
-        L *= R;
-      }
+      ffx_stage_tables(ax, tab);
     }
     nnative += fg.native ? 1 : 0;
     S.grp.push_back(fg);
@@ -318,8 +325,8 @@ int ffx_build(FfxSet& S, int ndim, const std::vector<SliceGeom>& hsl, const std:
 }
 
 int ffx_fwd(const FfxSet& S, const FfxGrid& G, PreMode mode, const float2* src, const float2* mps, float scale,
-            cudaStream_t st) {
-  for (int a = G.ndim - 1; a >= 0; --a)
+            cudaStream_t st, int first_axis) {
+  for (int a = G.ndim - 1; a >= first_axis; --a)
     for (const FfxStep& step : S.step[a]) {
       const int rc = a < G.ndim - 1 ? launch_pass<false, kFfxGrid, false>(S, G, step, nullptr, nullptr, nullptr, scale, st)
                      : mode == kPreSense
@@ -330,8 +337,8 @@ int ffx_fwd(const FfxSet& S, const FfxGrid& G, PreMode mode, const float2* src, 
   return MRN_OK;
 }
 
-int ffx_inv(const FfxSet& S, const FfxGrid& G, float2* out, float scale, cudaStream_t st) {
-  for (int a = 0; a < G.ndim; ++a)
+int ffx_inv(const FfxSet& S, const FfxGrid& G, float2* out, float scale, cudaStream_t st, int first_axis) {
+  for (int a = first_axis; a < G.ndim; ++a)
     for (const FfxStep& step : S.step[a]) {
       const int rc = a == G.ndim - 1 && out
                          ? launch_pass<true, kFfxGrid, true>(S, G, step, nullptr, nullptr, out, scale, st)

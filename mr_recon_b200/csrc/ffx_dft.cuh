@@ -198,6 +198,11 @@ __device__ __forceinline__ void dft(float2 (&x)[R]) {
   }
 }
 
+// Rows that a first-stage butterfly's R points take in shared memory: an odd
+// number, so lanes that run along the axis store without bank conflicts (512 =
+// 8 x 8 x 8 from the image: 8-way before).
+__host__ __device__ __forceinline__ int ffx_block_rows(int R) { return R | 1; }
+
 // What a pass reads first and writes last.
 enum FfxSrc { kFfxGrid = 0, kFfxImage = 1, kFfxSense = 2 };
 

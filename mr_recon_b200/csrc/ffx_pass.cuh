@@ -38,7 +38,7 @@ k_ffx_pass(const SliceGeom* __restrict__ sl, const FfxSlice* __restrict__ list, 
   if (f0 >= ncols) return;
   const int n = ps.ax.n, tid = threadIdx.x, nt = blockDim.x;
   const int R0 = ps.ax.radix[0], ns = ps.ax.ns;
-  const int r0s = R0 + ((ns == 2 && !(R0 & 1)) ? 1 : 0);  // odd row stride of the first stage's blocks
+  const int r0s = ffx_block_rows(R0);  // odd row stride of the first stage's blocks
   float2* tw = fsm;
   float2* A = fsm + n;
   float2* B = A + (size_t)(n / R0) * r0s * WS;  // used from three stages on
@@ -111,16 +111,17 @@ k_ffx_pass(const SliceGeom* __restrict__ sl, const FfxSlice* __restrict__ list, 
     }
   };
   // middle stage: shared -> shared
-  auto middle = [&](auto rc, const float2* a, float2* d, int s, int L) {
+  auto middle = [&](auto rc, const float2* a, float2* d, int s, int L, int rs) {
     constexpr int R = decltype(rc)::value;
     const int nr = n / R;
+    const int tstep = nr / L * rs;  // rs: rows of a block of L points
     const float2* tws = tw + ps.ax.tw_off[s];
     for (int idx = tid; idx < nr * W; idx += nt) {
       const int b = idx / W, w = idx - b * W;
       const int k = (int)__umulhi((unsigned)b, ps.ax.mag_l[s]), j = b - k * L;
       float2 x[R];
 #pragma unroll
-      for (int t = 0; t < R; ++t) x[t] = a[(b + t * nr) * WS + w];
+      for (int t = 0; t < R; ++t) x[t] = a[(k * rs + j + t * tstep) * WS + w];
 #pragma unroll
       for (int t = 1; t < R; ++t) x[t] = ctw<INV>(x[t], tws[j * (R - 1) + t - 1]);
       dft<R, INV>(x);
@@ -200,21 +201,21 @@ k_ffx_pass(const SliceGeom* __restrict__ sl, const FfxSlice* __restrict__ list, 
     const int R = ps.ax.radix[s];
     // radices above 12 come in two-stage lengths or first and last
     switch (R) {
-      case 2: middle(std::integral_constant<int, 2>(), A, B, s, L); break;
-      case 3: middle(std::integral_constant<int, 3>(), A, B, s, L); break;
-      case 4: middle(std::integral_constant<int, 4>(), A, B, s, L); break;
-      case 5: middle(std::integral_constant<int, 5>(), A, B, s, L); break;
-      case 6: middle(std::integral_constant<int, 6>(), A, B, s, L); break;
+      case 2: middle(std::integral_constant<int, 2>(), A, B, s, L, s == 1 ? r0s : L); break;
+      case 3: middle(std::integral_constant<int, 3>(), A, B, s, L, s == 1 ? r0s : L); break;
+      case 4: middle(std::integral_constant<int, 4>(), A, B, s, L, s == 1 ? r0s : L); break;
+      case 5: middle(std::integral_constant<int, 5>(), A, B, s, L, s == 1 ? r0s : L); break;
+      case 6: middle(std::integral_constant<int, 6>(), A, B, s, L, s == 1 ? r0s : L); break;
       case 7:
-        if constexpr (PRIMES) middle(std::integral_constant<int, 7>(), A, B, s, L);
+        if constexpr (PRIMES) middle(std::integral_constant<int, 7>(), A, B, s, L, s == 1 ? r0s : L);
         break;
       case 11:
-        if constexpr (PRIMES) middle(std::integral_constant<int, 11>(), A, B, s, L);
+        if constexpr (PRIMES) middle(std::integral_constant<int, 11>(), A, B, s, L, s == 1 ? r0s : L);
         break;
-      case 8: middle(std::integral_constant<int, 8>(), A, B, s, L); break;
-      case 9: middle(std::integral_constant<int, 9>(), A, B, s, L); break;
-      case 10: middle(std::integral_constant<int, 10>(), A, B, s, L); break;
-      default: middle(std::integral_constant<int, 12>(), A, B, s, L); break;
+      case 8: middle(std::integral_constant<int, 8>(), A, B, s, L, s == 1 ? r0s : L); break;
+      case 9: middle(std::integral_constant<int, 9>(), A, B, s, L, s == 1 ? r0s : L); break;
+      case 10: middle(std::integral_constant<int, 10>(), A, B, s, L, s == 1 ? r0s : L); break;
+      default: middle(std::integral_constant<int, 12>(), A, B, s, L, s == 1 ? r0s : L); break;
     }
     __syncthreads();
     float2* t = A;
@@ -240,8 +241,11 @@ int launch_ffx_pass(const FfxSet& S, const FfxGrid& G, const FfxStep& step, cons
   auto kern = k_ffx_pass<INV, SRC, TO_IMAGE, W, LIST, PRIMES>;
   const int rc = set_dynamic_smem(kern, step.smem);
   if (rc != MRN_OK) return rc;
+  // image and coil map take 94 registers a thread: above 320 threads one CTA
+  // would hold the SM alone
+  const int threads = SRC == kFfxSense && step.threads > 320 ? 256 : step.threads;
   for (int s0 = 0; s0 < step.nsl; s0 += 65535)
-    kern<<<dim3(nb, (unsigned)std::min(65535, step.nsl - s0)), step.threads, step.smem, st>>>(
+    kern<<<dim3(nb, (unsigned)std::min(65535, step.nsl - s0)), threads, step.smem, st>>>(
         G.dsl, S.d_list + step.first + s0, S.d_pass, step.pass, S.d_tw, G.grid, G.apod, src, mps, scale, out);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? MRN_OK : cuda_fail(e);

@@ -93,6 +93,10 @@ enum PreMode { kPrePlain = 0, kPreSense = 1 };
 int launch_pre(mrn_plan* P, PreMode mode, const float2* src, const float2* mps, float scale,
                cudaStream_t st);
 enum PostMode { kPostPlain = 0, kPostSense = 1 };
+// The SENSE combination of launch_post for any grid of the plan's images.
+int launch_post_sense(mrn_plan* P, const SliceGeom* dsl, const float* apod, const float2* grid, const float2* mps,
+                      float2* out, float scale, const float2* xin, float lam, double* pap, int pap_stride,
+                      unsigned* counter, cudaStream_t st);
 int launch_post(mrn_plan* P, PostMode mode, const float2* mps, float2* out, float scale,
                 const float2* xin, float lam, double* pap, int pap_stride, cudaStream_t st);
 int launch_shift_copy(mrn_plan* P, const float2* src, float2* dst, int to_user, cudaStream_t st);
@@ -139,9 +143,16 @@ void ffx_conv_tables(FfxAxis& ax, std::vector<float2>& tab);
 void ffx_conv_shape(FfxStep& st, const std::vector<FfxPass>& passes, int64_t total_cols, int sm_count);
 int launch_ffx_conv(const FfxSet& S, const FfxGrid& G, const FfxStep& step, bool inv, int source, bool to_image,
                     const float2* src, const float2* mps, float2* out, float scale, cudaStream_t st);
+// Forward / inverse transform of the axes from first_axis on.
 int ffx_fwd(const FfxSet& S, const FfxGrid& G, PreMode mode, const float2* src, const float2* mps, float scale,
-            cudaStream_t st);
-int ffx_inv(const FfxSet& S, const FfxGrid& G, float2* out, float scale, cudaStream_t st);
+            cudaStream_t st, int first_axis = 0);
+int ffx_inv(const FfxSet& S, const FfxGrid& G, float2* out, float scale, cudaStream_t st, int first_axis = 0);
+bool ffx_has_primes(const FfxAxis& ax);
+void ffx_stage_tables(FfxAxis& ax, std::vector<float2>& tab);
+// Forward FFT, kernel product and inverse FFT along the first axis (ffxturn.cu).
+int ffx_turn_build(FfxTurnSet& S, const FfxSet& F, int ndim, const std::vector<SliceGeom>& hsl,
+                   const std::vector<int64_t>& kern_off, int sm_count);
+int ffx_turn(const FfxTurnSet& S, const FfxGrid& G, const float2* kern, cudaStream_t st);
 int ffx_setup(mrn_plan* P);
 int ffx_refresh(mrn_plan* P);  // slice flags after MRN_OPT_NATIVE_FFT changes
 bool ffx_active(const mrn_plan* P);
