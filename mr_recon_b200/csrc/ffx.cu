@@ -350,23 +350,34 @@ int ffx_inv(const FfxSet& S, const FfxGrid& G, float2* out, float scale, cudaStr
 
 bool ffx_active(const mrn_plan* P) { return P->ffx.ok && P->use_ffx; }
 
-// Per-slice layout: a slice whose group runs the native passes (k_pre / k_post
-// leave it alone) has its grid in coil blocks, centred; the others keep coil
-// planes in FFT order.
-int ffx_refresh(mrn_plan* P) {
-  if (P->h_slices.empty() || !P->d_slices) return MRN_OK;
-  const int D = P->ndim;
-  for (auto& g : P->h_slices) {
-    g.native_fft = 0;
-    if (P->use_ffx)
-      for (const auto& fg : P->ffx.grp) {
-        bool same = fg.native;
-        for (int i = 0; i < D && same; ++i) same = g.nos[i] == fg.ax[i].n;
-        if (same) g.native_fft = 1;
-      }
-    g.cb = g.native_fft ? coil_block(g.ncoil) : 1;
-    for (int i = 0; i < D; ++i) g.hshift[i] = g.native_fft || (P->flags & MRN_PLAN_RAW) ? 0 : g.nos[i] / 2;
+// Lay the slices' grids out in d_grid, group by group: native groups in coil
+// blocks, centred, each slice from a multiple of 8 elements on (the
+// interpolation copies 16 bytes at a time, and the grids before it may have
+// any number of points); the others as coil planes in FFT order, back to back
+// for one batched cuFFT call. Returns the elements that takes.
+static int64_t place_grids(mrn_plan* P, bool use_native) {
+  int64_t off = 0;
+  for (size_t q = 0; q < P->fft.size(); ++q) {
+    auto& fg = P->fft[q];
+    const bool native = use_native && P->ffx.ok && P->ffx.grp[q].native;
+    off = (off + 7) / 8 * 8;
+    fg.grid_off = off;
+    for (int s : fg.slices) {
+      SliceGeom& g = P->h_slices[s];
+      g.native_fft = native ? 1 : 0;
+      g.cb = native ? coil_block(g.ncoil) : 1;
+      for (int i = 0; i < P->ndim; ++i) g.hshift[i] = native ? 0 : g.nos[i] / 2;
+      if (native) off = (off + 7) / 8 * 8;
+      g.grid_off = off;
+      off += (int64_t)((g.ncoil + g.cb - 1) / g.cb) * g.cb * g.gos;
+    }
   }
+  return off;
+}
+
+int ffx_refresh(mrn_plan* P) {
+  if (P->fft.empty() || !P->d_slices) return MRN_OK;
+  place_grids(P, P->use_ffx);
   return upload_slices(P) == cudaSuccess ? MRN_OK : MRN_ERR_CUDA;
 }
 
@@ -382,6 +393,9 @@ int ffx_setup(mrn_plan* P) {
   }
   const int rc = ffx_build(P->ffx, P->ndim, P->h_slices, spec, P->use_conv, P->sm_count);
   if (rc != MRN_OK) return rc;
+  // room for either value of MRN_OPT_NATIVE_FFT
+  P->n_igrid = place_grids(P, false);
+  P->n_igrid = std::max(P->n_igrid, place_grids(P, true));
   return ffx_refresh(P);
 }
 

@@ -633,9 +633,8 @@ int mrn_plan_create(mrn_plan** out, int ndim, int n_slices, const int* im_size,
     P->coil_group = std::max(1, cg);
   }
 
-  // FFT groups in first-seen order; internal grid buffer ordered by group.
+  // FFT groups (one grid size each) in first-seen order; the internal grid buffer is ordered by group.
   if (!raw) {
-    std::vector<int> group_of(n_slices, -1);
     for (int s = 0; s < n_slices; ++s) {
       const SliceGeom& g = P->h_slices[s];
       int found = -1;
@@ -652,7 +651,8 @@ int mrn_plan_create(mrn_plan** out, int ndim, int n_slices, const int* im_size,
         P->fft.push_back(fg);
         found = (int)P->fft.size() - 1;
       }
-      group_of[s] = found;
+      P->fft[found].slices.push_back(s);
+      P->fft[found].batch += g.ncoil;
     }
     // Chirp convolutions pay where cuFFT would stream the grid from HBM several
     // times or run grid sizes one after the other: from a million points, or
@@ -662,23 +662,6 @@ int mrn_plan_create(mrn_plan** out, int ndim, int n_slices, const int* im_size,
     int64_t points = 0;
     for (const SliceGeom& g : P->h_slices) points += (int64_t)g.ncoil * g.gos;
     P->use_conv = P->fft.size() > 1 || points >= 1000000;
-    // grids that can run the native passes hold whole coil blocks; with
-    // MRN_OPT_NATIVE_FFT 0 their unused coils are transformed along
-    int64_t off = 0;
-    for (size_t q = 0; q < P->fft.size(); ++q) {
-      P->fft[q].grid_off = off;
-      const bool can = ffx_can(ndim, P->fft[q].nos, P->use_conv);
-      for (int s = 0; s < n_slices; ++s)
-        if (group_of[s] == (int)q) {
-          SliceGeom& g = P->h_slices[s];
-          const int cb = can ? coil_block(g.ncoil) : 1;
-          const int padded = (g.ncoil + cb - 1) / cb * cb;
-          g.grid_off = off;
-          off += (int64_t)padded * g.gos;
-          P->fft[q].batch += padded;
-        }
-    }
-    P->n_igrid = off;
   } else {
     for (int s = 0; s < n_slices; ++s) P->h_slices[s].grid_off = P->h_slices[s].ugrid_off;
   }
@@ -743,9 +726,9 @@ int mrn_plan_create(mrn_plan** out, int ndim, int n_slices, const int* im_size,
   PK(dev_alloc(&P->d_red, (size_t)n_slices * kMaxRedBlocks));
   PK(dev_alloc(&P->d_rowpart, (size_t)std::max<int64_t>(P->n_xrow, 1)));
   if (!raw) {
+    PK(ffx_setup(P));
     PK(dev_alloc(&P->d_grid, std::max<int64_t>(P->n_igrid, 1)));
     PK(dev_alloc(&P->d_ksp_tmp, std::max<int64_t>(P->n_ksp, 1)));
-    PK(ffx_setup(P));
     PK(cufft_setup(P));
   }
   PK(gather_setup(P));
