@@ -126,8 +126,7 @@ constexpr int kFfxMaxStages = 4;
 constexpr int kFfxMaxN = 1024;
 // Lengths with a prime factor above 5 run natively from here on. Shorter grids
 // are launch-bound either way and keep cuFFT (78^2 image, 98^2 grid, 8 coils:
-// FFT stage with pad and crop 50 us natively, 49 with cuFFT; 97 x 109, 4 coils:
-// 47 and 63; 203^2, 32 coils: 151 and 298).
+// FFT stage with pad and crop 50 us natively, 49 with cuFFT).
 constexpr int kFfxConvMin = 96;
 struct FfxAxis {
   int n;
@@ -171,12 +170,12 @@ struct FfxStep {
   size_t smem;
 };
 
-// One FFT group of a grid buffer (slices of one grid size). native: its slices
-// have the same image size and every axis has a plan (ffx_axis).
+// One FFT group of a grid buffer (slices of one grid and image size). native:
+// every axis has a plan (ffx_axis).
 struct FfxGroup {
   bool native;
   FfxAxis ax[kMaxDim];
-  int first_slice;  // geometry (image and grid size) shared by the group's slices
+  std::vector<int> slices;
 };
 
 // The native FFT of one grid buffer: its groups, the launches of each axis,
@@ -543,9 +542,11 @@ struct mrn_plan {
   unsigned* d_sync = nullptr;       // last-block counters: [0] k_cg_dir, [1] CG sums, [2] k_post
   double* d_red = nullptr;          // CG block partial sums, [n_slices][kMaxRedBlocks]
   double* d_rowpart = nullptr;      // k_post per-row partials of Re<x, out>, [n_xrow]
-  // FFT groups: slices with identical Nos share one batched cuFFT plan
+  // FFT groups: slices with identical Nos that are transformed the same way
   struct FftGroup {
     int nos[mrn::kMaxDim];
+    bool native;        // by the native passes (ffx_pays), while MRN_OPT_NATIVE_FFT is on; else
+                        // by one batched cuFFT plan
     int64_t grid_off;   // complex offset in d_grid
     int batch;          // sum of coils
     cufftHandle handle;
@@ -556,7 +557,6 @@ struct mrn_plan {
   // selects it (default) or cuFFT for every group.
   mrn::FfxSet ffx;
   bool use_ffx = true;
-  bool use_conv = false;  // axes without direct radices may run as chirp convolutions
   // Interpolation from the grid in coil blocks (gather.cu): the slices of
   // each block width, cut into CTAs of `chunk` sorted samples.
   struct GatherSet {

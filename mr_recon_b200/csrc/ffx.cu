@@ -107,8 +107,37 @@ bool ffx_factor(int n, FfxAxis& ax) {
   return true;
 }
 
-// Direct radices, or (conv) a chirp convolution from kFfxConvMin points on.
-bool ffx_axis(int n, bool conv, FfxAxis& ax) { return ffx_factor(n, ax) || (conv && ffx_conv_axis(n, ax)); }
+// Direct radices where the length has them, else a chirp convolution.
+bool ffx_axis(int n, FfxAxis& ax) { return ffx_factor(n, ax) || ffx_conv_axis(n, ax); }
+
+// Whether an axis of a plan grid of `points` values, `least` along its shortest
+// axis, is worth a native pass beside cuFFT with separate pad and crop. Times:
+// forward + adjoint with 64 samples, natively and with cuFFT.
+// - products of 2, 3 and 5: always.
+// - factors 7 to 19: in two stages (323^2, 16 coils: 85 and 97 us; 132^3, 8
+//   coils: 0.55 and 0.72 ms). A third stage at these kernels' 90 registers loses
+//   (408^2, 32 coils: 272 and 203 us; 175^3, 8 coils: 2.47 and 1.79 ms) unless the
+//   grid is so small that launches dominate (338^2, 1 coil: 55 and 57 us; 1001 x
+//   10, 8 coils: 56 and 59).
+// - chirp convolutions from 0.7 M points (326^2, 4 coils, 0.43 M: 89 and 83 us;
+//   272 x 326, 7, 0.62 M: 92 and 88; 394^2, 4, 0.62 M: 94 and 101; 303^2, 8, 0.73 M:
+//   107 and 137; 254^2, 32, 2.1 M: 166 and 298; 146^3, 8: 1.83 and 3.45 ms) and for slabs, a few short
+//   launches either way (163 x 10, 3 coils: 61 and 59; 401 x 10: 68 and 51), where
+//   the largest prime is above 31: cuFFT is fast on the smaller ones (464 = 16 x
+//   29, 32 coils: 446 and 181 us; 217^3, 4 coils: 4.2 and 2.9 ms). Not for prime
+//   lengths from 201 to 256: their convolutions of 480 and 512 points take
+//   radices 24 and 32, which leave fewer warps an SM (227^2, 32 coils: 157 and
+//   137 us; 257^2, 32: 171 and 210).
+bool ffx_axis_pays(int n, int64_t points, int least) {
+  FfxAxis ax;
+  if (ffx_factor(n, ax)) return !ffx_has_primes(ax) || ax.ns == 2 || points < 200000;
+  if ((points < 700000 && least > 20) || !ffx_conv_axis(n, ax)) return false;
+  int p = 2, m = n;
+  while (p * p <= m)
+    if (m % p == 0) m /= p;
+    else ++p;
+  return m > 31 && !(m == n && n > 200 && n <= 256);
+}
 
 template <class T>
 int upload(T** dst, const std::vector<T>& v) {
@@ -199,21 +228,36 @@ void ffx_stage_tables(FfxAxis& ax, std::vector<float2>& tab) {
   }
 }
 
-// Whether every axis of a grid can run the native passes.
-bool ffx_can(int ndim, const int* nos, bool conv) {
+// Whether every axis of a grid has direct radices.
+bool ffx_direct(int ndim, const int* nos) {
   if (ndim != 2 && ndim != 3) return false;
   FfxAxis ax;
   for (int i = 0; i < ndim; ++i)
-    if (!ffx_axis(nos[i], conv, ax)) return false;
+    if (!ffx_factor(nos[i], ax)) return false;
   return true;
 }
 
-// Build the native FFT of a grid buffer: per group spec (grid size) its axes'
-// plans and tables, and per axis the lists of slices that run together. A
-// group whose slices differ in image size, or with an axis that has no plan,
-// is not native.
+// Whether a slice of a plan grid runs the native passes: by its own grid and
+// coils alone, so that it is transformed the same way (the same bits) whatever
+// shares its plan.
+bool ffx_pays(int ndim, const int* nos, int ncoil) {
+  if (ndim != 2 && ndim != 3) return false;
+  int64_t points = ncoil;
+  int least = nos[0];
+  for (int i = 0; i < ndim; ++i) {
+    points *= nos[i];
+    least = std::min(least, nos[i]);
+  }
+  for (int i = 0; i < ndim; ++i)
+    if (!ffx_axis_pays(nos[i], points, least)) return false;
+  return true;
+}
+
+// Build the native FFT of a grid buffer: per native group its axes' plans and
+// tables, and per axis the lists of slices that run together. The slices of a
+// group have one grid and one image size.
 int ffx_build(FfxSet& S, int ndim, const std::vector<SliceGeom>& hsl, const std::vector<FfxGroupSpec>& spec,
-              bool conv, int sm_count) {
+              int sm_count) {
   S.release();
   if ((ndim != 2 && ndim != 3) || hsl.empty()) return MRN_OK;
   const int D = ndim;
@@ -221,21 +265,11 @@ int ffx_build(FfxSet& S, int ndim, const std::vector<SliceGeom>& hsl, const std:
   int nnative = 0;
   for (const FfxGroupSpec& gs : spec) {
     FfxGroup fg{};
-    fg.native = true;
-    fg.first_slice = -1;
-    for (int s = 0; s < (int)hsl.size(); ++s) {
-      const SliceGeom& g = hsl[s];
-      bool same = true;
-      for (int i = 0; i < D; ++i) same &= g.nos[i] == gs.nos[i];
-      if (!same) continue;
-      if (fg.first_slice < 0) fg.first_slice = s;
-      const SliceGeom& g0 = hsl[fg.first_slice];
-      for (int i = 0; i < D; ++i) fg.native &= g.n[i] == g0.n[i];
-    }
-    if (fg.first_slice < 0) fg.native = false;
+    fg.native = gs.native;
+    fg.slices = gs.slices;
     for (int i = 0; i < D && fg.native; ++i) {
       FfxAxis& ax = fg.ax[i];
-      if (!ffx_axis(gs.nos[i], conv, ax)) {
+      if (!ffx_axis(hsl[gs.slices[0]].nos[i], ax)) {
         fg.native = false;
         break;
       }
@@ -276,7 +310,7 @@ int ffx_build(FfxSet& S, int ndim, const std::vector<SliceGeom>& hsl, const std:
       int64_t total = 0;
       for (const FfxGroup& fg : S.grp) {
         if (!fg.native || (fg.ax[a].m > 0 ? 2 : (int)has_primes(fg.ax[a])) != kind) continue;
-        const SliceGeom& g0 = hsl[fg.first_slice];
+        const SliceGeom& g0 = hsl[fg.slices[0]];
         FfxPass ps{};
         ps.ax = fg.ax[a];
         ps.axis = a;
@@ -289,11 +323,9 @@ int ffx_build(FfxSet& S, int ndim, const std::vector<SliceGeom>& hsl, const std:
         for (int narrow = 0; narrow < 2; ++narrow) {  // a group's slices by the width of their coil blocks
           bool used = false;
           ps.narrow = narrow;
-          for (int s = 0; s < (int)hsl.size(); ++s) {
-            bool same = true;
-            for (int i = 0; i < D; ++i) same &= hsl[s].nos[i] == g0.nos[i];
+          for (int s : fg.slices) {
             const int cb = coil_block(hsl[s].ncoil);
-            if (!same || (a == D - 1 && cb < 8) != (narrow != 0)) continue;
+            if ((a == D - 1 && cb < 8) != (narrow != 0)) continue;
             used = true;
             list.push_back(FfxSlice{s, (int)passes.size()});
             const int64_t cols = (int64_t)hsl[s].ncoil * ps.pcols * ps.icells;
@@ -386,12 +418,8 @@ int ffx_setup(mrn_plan* P) {
   P->ffx.release();
   if (P->flags & MRN_PLAN_RAW) return MRN_OK;
   std::vector<FfxGroupSpec> spec;
-  for (const auto& f : P->fft) {
-    FfxGroupSpec gs{};
-    for (int i = 0; i < kMaxDim; ++i) gs.nos[i] = f.nos[i];
-    spec.push_back(gs);
-  }
-  const int rc = ffx_build(P->ffx, P->ndim, P->h_slices, spec, P->use_conv, P->sm_count);
+  for (const auto& f : P->fft) spec.push_back(FfxGroupSpec{f.native, f.slices});
+  const int rc = ffx_build(P->ffx, P->ndim, P->h_slices, spec, P->sm_count);
   if (rc != MRN_OK) return rc;
   // room for either value of MRN_OPT_NATIVE_FFT
   P->n_igrid = place_grids(P, false);

@@ -117,11 +117,12 @@ int inv_transform(mrn_plan* P, float2* out, cudaStream_t st);
 // Slice table upload (plan.cu): d_slices and its shared-k-space twin.
 cudaError_t upload_slices(mrn_plan* P);
 
-// Native FFT (ffx.cu). A grid buffer of FFT groups, each one grid size;
-// FfxGrid is what the passes read (host and device slice tables,
+// Native FFT (ffx.cu). A grid buffer of FFT groups, each the slices of one grid
+// and image size; FfxGrid is what the passes read (host and device slice tables,
 // apodization, the buffer).
 struct FfxGroupSpec {
-  int nos[kMaxDim];
+  bool native;  // run the native passes if every axis has a plan
+  std::vector<int> slices;
 };
 struct FfxGrid {
   int ndim;
@@ -131,9 +132,10 @@ struct FfxGrid {
   float2* grid;
   int sm_count;
 };
-bool ffx_can(int ndim, const int* nos, bool conv);  // every axis of the grid size can run natively
+bool ffx_direct(int ndim, const int* nos);            // every axis has direct radices
+bool ffx_pays(int ndim, const int* nos, int ncoil);  // the native passes of a plan grid are worth it
 int ffx_build(FfxSet& S, int ndim, const std::vector<SliceGeom>& hsl, const std::vector<FfxGroupSpec>& spec,
-              bool conv, int sm_count);
+              int sm_count);
 // Direct passes with radices 7, 11, 13, 14, 17, 19 (ffxprime.cu).
 int launch_ffx_primes(const FfxSet& S, const FfxGrid& G, const FfxStep& step, bool inv, int source, bool to_image,
                       const float2* src, const float2* mps, float2* out, float scale, cudaStream_t st);

@@ -633,19 +633,21 @@ int mrn_plan_create(mrn_plan** out, int ndim, int n_slices, const int* im_size,
     P->coil_group = std::max(1, cg);
   }
 
-  // FFT groups (one grid size each) in first-seen order; the internal grid buffer is ordered by group.
+  // FFT groups (one grid size, one way to transform it) in first-seen order; the internal grid buffer is ordered by group.
   if (!raw) {
     for (int s = 0; s < n_slices; ++s) {
       const SliceGeom& g = P->h_slices[s];
+      const bool native = ffx_pays(ndim, g.nos, g.ncoil);
       int found = -1;
       for (size_t q = 0; q < P->fft.size(); ++q) {
-        bool same = true;
+        bool same = P->fft[q].native == native;
         for (int i = 0; i < ndim; ++i) same &= (P->fft[q].nos[i] == g.nos[i]);
         if (same) { found = (int)q; break; }
       }
       if (found < 0) {
         mrn_plan::FftGroup fg{};
         for (int i = 0; i < kMaxDim; ++i) fg.nos[i] = g.nos[i];
+        fg.native = native;
         fg.batch = 0;
         fg.handle = 0;
         P->fft.push_back(fg);
@@ -654,14 +656,6 @@ int mrn_plan_create(mrn_plan** out, int ndim, int n_slices, const int* im_size,
       P->fft[found].slices.push_back(s);
       P->fft[found].batch += g.ncoil;
     }
-    // Chirp convolutions pay where cuFFT would stream the grid from HBM several
-    // times or run grid sizes one after the other: from a million points, or
-    // for several sizes (one 272 x 326 grid of 7 coils, 0.6 M: forward + adjoint
-    // 92 us with them, 87 with cuFFT; 254^2, 32 coils, 2.1 M: FFT stage 149
-    // and 298; 142 x 195 x 152, 6 coils, 25 M: 1.28 ms and 2.24)
-    int64_t points = 0;
-    for (const SliceGeom& g : P->h_slices) points += (int64_t)g.ncoil * g.gos;
-    P->use_conv = P->fft.size() > 1 || points >= 1000000;
   } else {
     for (int s = 0; s < n_slices; ++s) P->h_slices[s].grid_off = P->h_slices[s].ugrid_off;
   }

@@ -381,21 +381,22 @@ static bool toep_native(mrn_plan* P, ToepState* T) {
   for (int s = 0; s < P->nslices; ++s) {
     SliceGeom& g = T->hsl[s];
     const ToepGeom& t = T->h[s];
-    if (!ffx_can(D, t.np, false)) return false;
-    FfxGroupSpec gs{};
+    if (!ffx_direct(D, t.np)) return false;
     for (int i = 0; i < kMaxDim; ++i) {
-      g.nos[i] = gs.nos[i] = t.np[i];
+      g.nos[i] = t.np[i];
       g.hshift[i] = 0;
       g.apod_off[i] = 0;
       longest = std::max(longest, t.n[i]);
     }
-    bool seen = false;
-    for (const auto& o : spec) {
+    FfxGroupSpec* gs = nullptr;  // slices of one padded and one image size
+    for (auto& o : spec) {
+      const SliceGeom& f = T->hsl[o.slices[0]];
       bool eq = true;
-      for (int i = 0; i < D; ++i) eq &= o.nos[i] == gs.nos[i];
-      seen |= eq;
+      for (int i = 0; i < D; ++i) eq &= f.nos[i] == g.nos[i] && f.n[i] == g.n[i];
+      if (eq) gs = &o;
     }
-    if (!seen) spec.push_back(gs);
+    if (gs) gs->slices.push_back(s);
+    else spec.push_back(FfxGroupSpec{true, {s}});
     g.gos = t.gp;
     g.native_fft = 1;
     g.cb = coil_block(g.ncoil);
@@ -404,7 +405,7 @@ static bool toep_native(mrn_plan* P, ToepState* T) {
     off += (int64_t)((g.ncoil + g.cb - 1) / g.cb) * g.cb * t.gp;
     kern_off.push_back(t.kern_off);
   }
-  if (ffx_build(T->ffx, D, T->hsl, spec, false, P->sm_count) != MRN_OK || !T->ffx.all ||
+  if (ffx_build(T->ffx, D, T->hsl, spec, P->sm_count) != MRN_OK || !T->ffx.all ||
       ffx_turn_build(T->turn, T->ffx, D, T->hsl, kern_off, P->sm_count) != MRN_OK) {
     T->ffx.release();
     T->turn.release();

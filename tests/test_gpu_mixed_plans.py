@@ -57,3 +57,34 @@ def test_grids_start_on_whole_sectors(ims, ms, coils):
         plan = Plan(ims, ms, coils, 1.25, (6.0, 6.0), device=DEV)
         plan.set_option(_lib.MRN_OPT_NATIVE_FFT, native)
         _check(plan, ims, ms, coils, 1.25, 6.0, np.random.RandomState(len(ims) + ms[0]))
+
+
+@pytest.mark.parametrize("ims,coils", [
+    ([(203, 203), (163, 150), (64, 64), (181, 217), (331, 150), (203, 203)], [4, 8, 1, 7, 3, 32]),
+    ([(82, 20, 24), (48, 48, 48), (82, 96, 80)], [3, 5, 8]),
+])
+def test_transforms_do_not_depend_on_the_other_slices(ims, coils):
+    """Grids with large prime factors (254 = 2 x 127, 326 = 2 x 163, 103) beside others, the same size with few and
+    with many coils: each slice's transforms have the bits that they have in a plan of their own."""
+    from mr_recon_b200.plan import Plan
+    rng = np.random.RandomState(len(ims))
+    d = len(ims[0])
+
+    def transforms(ims, coils, img, src):
+        p = Plan(ims, [0] * len(ims), coils, 1.25, (4.0,) * d, device=DEV)
+        grid, back = torch.empty_like(src), torch.empty_like(img)
+        p.forward_ft(img, grid)
+        p.adjoint_ift(src, back)
+        return p, grid, back
+
+    n_img = [c * int(np.prod(im)) for im, c in zip(ims, coils)]
+    n_grid = [c * int(np.prod([-(-5 * n // 4) for n in im])) for im, c in zip(ims, coils)]
+    img = torch.from_numpy(_cplx(rng, (sum(n_img),))).to(DEV)
+    src = torch.from_numpy(_cplx(rng, (sum(n_grid),))).to(DEV)
+    both, grid, back = transforms(ims, coils, img, src)
+    for s in range(len(ims)):
+        i = slice(int(both.img_off[s]), int(both.img_off[s]) + n_img[s])
+        g = slice(int(both.grid_off[s]), int(both.grid_off[s]) + n_grid[s])
+        _, one_grid, one_back = transforms([ims[s]], [coils[s]], img[i].contiguous(), src[g].contiguous())
+        assert torch.equal(grid[g], one_grid), f"forward, slice {s}"
+        assert torch.equal(back[i], one_back), f"inverse, slice {s}"
