@@ -132,3 +132,57 @@ def test_register_tile_gridding(im, os_, W, C, chunk):
     assert _rel(g.cpu().numpy(), on.adjoint_grid_only(ksp[None], trj[None])[0]) < 1e-5
     x = torch.from_numpy((rng.randn(*im) + 1j * rng.randn(*im)).astype(np.complex64)).to(DEV)
     assert torch.equal(A.normal(x), A.adjoint(A.forward(x)))
+
+
+# (lengths of the grid, coils): lengths with factors 11 to 19, or a large prime, with columns enough for the widest CTAs (16
+# direct, 8 as a chirp convolution), on each axis, in whole and ragged blocks of 8 coils
+WIDE = [((209, 323), 9), ((323, 209), 32), ((539, 40), 9), ((40, 616), 8), ((361, 96), 32), ((96, 361), 9),
+        ((206, 400), 9), ((100, 254), 32), ((254, 96), 33), ((401, 200), 9), ((180, 509), 17), ((509, 320), 32),
+        ((206, 50, 40), 9), ((50, 206, 40), 9), ((40, 50, 206), 11), ((254, 254, 30), 8), ((121, 48, 60), 17),
+        ((48, 121, 60), 9), ((48, 60, 121), 12)]
+
+
+@pytest.mark.parametrize("nos,C", WIDE)
+def test_wide_transforms(nos, C):
+    """Transforms of many columns against 64 bits, and the coil-map source and sum against the plain ones."""
+    from mr_recon_b200.plan import Plan
+    d = len(nos)
+    os_ = next(o for o in (1.25, 1.5, 1.375, 1.125, 1.0) if all(math.ceil(o * int(n / o)) == n for n in nos))
+    im = tuple(int(n / os_) for n in nos)
+    rng = np.random.RandomState(sum(nos) + C)
+    M = 300
+    p = Plan([im], [M], [C], os_, (4.0,) * d, beta=9.0, device=DEV)
+    assert tuple(p.os_sizes[0]) == nos and p.fft_kind == 1
+    cplx = lambda *s: (rng.randn(*s) + 1j * rng.randn(*s)).astype(np.complex64)  # noqa: E731
+    dev = lambda a: torch.from_numpy(a).to(DEV)  # noqa: E731
+    img, src = cplx(C, *im), cplx(C, *nos)
+    grid = torch.empty(src.shape, dtype=torch.complex64, device=DEV)
+    back = torch.empty(img.shape, dtype=torch.complex64, device=DEV)
+    p.forward_ft(dev(img), grid)
+    p.adjoint_ift(dev(src), back)
+    a = np.ones(())
+    for m, o in zip(im, nos):
+        t = np.sqrt(9.0 ** 2 - (np.pi * 4.0 * (np.arange(m) - m // 2) / o) ** 2 + 0j)
+        a = a[..., None] * (t / np.sinh(t)).real
+    a = a / math.sqrt(np.prod(im))
+    at = (slice(None),) + tuple(slice(o // 2 - m // 2, o // 2 - m // 2 + m) for m, o in zip(im, nos))
+    pad = np.zeros(src.shape, np.complex128)
+    pad[at] = img * a
+    ax = tuple(range(1, d + 1))
+    want = np.fft.fftshift(np.fft.fftn(np.fft.ifftshift(pad, axes=ax), axes=ax), axes=ax)
+    wback = np.fft.fftshift(np.fft.ifftn(np.fft.ifftshift(src.astype(np.complex128), axes=ax), axes=ax, norm="forward"),
+                            axes=ax)[at] * a
+    # float32 butterflies: a few ulp (6e-8) per stage, at most five stages an axis
+    assert _rel(grid.cpu().numpy(), want) < 1e-6
+    assert _rel(back.cpu().numpy(), wback) < 1e-6
+    p.set_traj(dev(((rng.rand(M, d) - 0.5) * np.array(im)).astype(np.float32).reshape(-1)))
+    x, mps = dev(cplx(*im)), dev(cplx(C, *im))
+    ks, kp = (torch.empty(C * M, dtype=torch.complex64, device=DEV) for _ in range(2))
+    p.sense_forward(x, mps, ks)
+    p.forward(mps * x, kp)
+    xs = torch.empty_like(x)
+    p.sense_adjoint(kp, None, mps, xs)
+    p.adjoint(kp, back)
+    # one rounding of the coil product (and of the sum of up to 33 coils) apart
+    assert _rel(ks.cpu().numpy(), kp.cpu().numpy()) < 1e-6
+    assert _rel(xs.cpu().numpy(), (mps.conj() * back).sum(0).cpu().numpy()) < 1e-6
