@@ -110,8 +110,8 @@ int mrn_plan_fft_kind(const mrn_plan* plan);
 /* Work decomposition (each takes effect at the next mrn_plan_set_traj):
  * MRN_OPT_INTERP_CHUNK / MRN_OPT_GRID_CHUNK: samples per interpolation work
  * item and gridding entries per gridding work item (defaults: 256 in 2D, 1024
- * in 3D and 1D; gridding: from the entry count, 64 to 256 in 2D, 512 to 4096
- * in 3D, 1024 in 1D); MRN_OPT_INTERP_TILE / MRN_OPT_GRID_TILE:
+ * in 3D and 1D; gridding: from each slice's own entry count, 96 to 256 in 2D,
+ * 512 to 4096 in 3D, 1024 in 1D); MRN_OPT_INTERP_TILE / MRN_OPT_GRID_TILE:
  * tile edge in grid cells, every dimension (defaults: 10 / 8 in 2D, 4 / 8 in
  * 3D, 256 in 1D). */
 #define MRN_OPT_INTERP_CHUNK 4

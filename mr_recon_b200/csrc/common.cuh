@@ -462,7 +462,7 @@ struct mrn_plan {
   int coil_group_req = 0;  // caller's coil group, 0 = choose per kernel kind
   int max_coil = 1;
   int max_chunk = 1024;   // samples per interpolation work item
-  int grid_chunk = 0;     // entries per gridding work item, 0 = from the entry count
+  int grid_chunk = 0;     // entries per gridding work item, 0 = from each slice's entry count
   int tap_max = 8;  // compile-time tap bound used (8 or 16)
   bool use_fast = true;  // use the unrolled fixed-K tile kernels where they apply
   mrn::KBParams kb{};
@@ -523,7 +523,8 @@ struct mrn_plan {
   int* d_tile_item_off = nullptr;
   mrn::Item* d_items_i = nullptr;
   mrn::Item* d_items_g = nullptr;
-  int* d_counts = nullptr;          // [0] n_items_i [1] n_items_g [2] n_entries_g [3] n_split
+  int2* d_slice_ent = nullptr;      // per slice {gridding entries, entries per gridding work item}
+  int* d_counts = nullptr;          // [0] n_items_i [1] n_items_g [3] n_split
                                     // [4] partial-tile slots in use
   int4* d_split_tiles = nullptr;    // split gridding tiles: {global tile, first slot, items, 0}
   float2* d_part = nullptr;         // partial tiles of split gridding tiles (SplitOut)

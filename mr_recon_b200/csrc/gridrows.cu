@@ -336,10 +336,15 @@ k_grid_rows(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KB
       bool meet = h32 + lane < nb;
       if (D == 3) meet &= ((mine >> (8 + (warp % NPG) * PPW)) & ((1u << PPW) - 1u)) != 0u;
       if (D == 3 || CW == 32) meet &= ((mine >> (16 + 4 * half)) & 15u) != 0u;
-      unsigned act = __ballot_sync(0xffffffffu, meet);
+      // windows in the order of all 32 entries, also those the warp skips: a
+      // cell's order does not depend on which planes share its warp (CW)
+      unsigned act = __ballot_sync(0xffffffffu, meet), left = 0xffffffffu;
       while (act) {
-        const int code = __shfl_sync(0xffffffffu, zcode, __ffs(act) - 1);
-        const unsigned same = __ballot_sync(0xffffffffu, zcode == code) & act;
+        const int code = __shfl_sync(0xffffffffu, zcode, __ffs(left) - 1);
+        unsigned same = __ballot_sync(0xffffffffu, zcode == code);
+        left &= ~same;
+        same &= act;
+        if (!same) continue;
         act &= ~same;
         RunBody<D, CW, B, TEMP> body{acc, s, b2, h32, plane, half, coil, stream, same};
         body.template dispatch<KW>(code);

@@ -179,19 +179,21 @@ __global__ void k_tile_hist(const unsigned* __restrict__ key, int64_t n, int* __
   if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(cnt + k, __popc(peers));
 }
 
-// Append the window code and, in tiles of more than `chunk` entries, the part
-// of the trajectory to the tile keys.
+// Append the window code and, in tiles of more entries than a work item of
+// their slice takes, the part of the trajectory to the tile keys.
 __global__ void k_entry_codes(const SliceGeom* __restrict__ sl, int ns, int ndim, KBParams kb,
                               const float4* __restrict__ coord, const int* __restrict__ val,
-                              const int* __restrict__ cnt, int chunk, int64_t n, unsigned* __restrict__ key) {
+                              const int* __restrict__ cnt, const int2* __restrict__ ent, int64_t n,
+                              unsigned* __restrict__ key) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
   const int t = (int)key[e], p = val[e];
-  const SliceGeom& g = sl[find_slice_by_tile(sl, ns, t, 1)];
+  const int s = find_slice_by_tile(sl, ns, t, 1);
+  const SliceGeom& g = sl[s];
   const int i = ndim - 1;
   const float4 c4 = coord[p];
   const unsigned code = (unsigned)window_code(g, kb, i == 2 ? c4.z : c4.y, (t - g.gtile_base) % g.gntile[i], i);
-  const unsigned part = cnt[t] > chunk ? (unsigned)(((int64_t)p - g.pt_off) * (1 << kGPartBits) / g.m) : 0u;
+  const unsigned part = cnt[t] > ent[s].y ? (unsigned)(((int64_t)p - g.pt_off) * (1 << kGPartBits) / g.m) : 0u;
   key[e] = (unsigned)t << kGCodeBits | part << kGWinBits | code;
 }
 
@@ -211,12 +213,16 @@ __global__ void k_tile_ranges(const unsigned* __restrict__ key, int code_bits, i
   if (e == n - 1 || key[e + 1] >> code_bits != k) end[k] = (int)(e + 1);
 }
 
-__global__ void k_item_counts(const int* __restrict__ start, const int* __restrict__ end,
-                              int ntiles, int chunk, int min_items, int* __restrict__ nitems) {
+// Items per tile: entries / chunk, rounded up (gridding: the chunk of the
+// tile's slice, and at least one item, which stores an empty tile's zeros).
+__global__ void k_item_counts(const SliceGeom* __restrict__ sl, int ns, const int2* __restrict__ ent,
+                              const int* __restrict__ start, const int* __restrict__ end,
+                              int ntiles, int chunk, int gridding, int* __restrict__ nitems) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ntiles) return;
   const int c = end[t] - start[t];
-  nitems[t] = max(min_items, (c + chunk - 1) / chunk);
+  const int k = gridding ? ent[find_slice_by_tile(sl, ns, t, 1)].y : chunk;
+  nitems[t] = max(gridding, (c + k - 1) / k);
 }
 
 // Work items of every tile at the scanned offsets. Gridding tiles with more
@@ -274,23 +280,35 @@ __global__ void k_gather_items(const Item* __restrict__ src, const int* __restri
   if (i < n) dst[i] = src[idx[i]];
 }
 
-__global__ void k_total(const int* __restrict__ off, const int* __restrict__ cnt, int64_t n,
-                        int* __restrict__ out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *out = n > 0 ? off[n - 1] + cnt[n - 1] : 0;
+// Gridding entries per work item of a slice: from its own entries alone, so that
+// a cell's sums are the same whatever shares the plan. About six items per SM in
+// 2D and four in 3D would share a slice's entries evenly; fewer entries leave
+// the densest tiles as a tail, more split tiles cost partial tiles. 2D 96..256
+// (256^2, 32 coils, 266 k entries: 64 / 128 / 192 / 256 / 512 entries 172 / 110 /
+// 91 / 87 / 111 us; 128^2, 1 coil, 50 k: 64 / 96 / 128 / 256 27.5 / 28.3 / 32 / 46,
+// but 16 such slices of 8 coils together 223 / 181 / 164 / 141), 3D 512..4096
+// (192^3, 16 coils, 20.6 M: 2048 / 4096 / 8192 6.1 / 5.8 / 5.7 ms; the last one's
+// longer partial sums near the k-space centre round more; 64^3, 8 coils, 0.7 M:
+// 512 / 1024 / 2048 / 4096 238 / 206 / 219 / 349 us, four such slices 909 / 718 /
+// 615 / 601).
+__host__ __device__ static int grid_chunk_of(int ndim, int sm_count, int64_t entries) {
+  if (ndim == 1) return 1024;
+  const int64_t lo = ndim == 2 ? 96 : 512, hi = ndim == 2 ? 256 : 4096;
+  const int64_t share = entries / ((ndim == 2 ? 6 : 4) * (int64_t)sm_count);
+  const int64_t c = (share + 31) / 32 * 32;
+  return (int)(c < lo ? lo : (c > hi ? hi : c));
 }
 
-// Gridding entries per work item: about six items per SM in 2D and four in 3D
-// would share E evenly; fewer entries leave the densest tiles as a tail, more
-// split tiles cost partial tiles. 2D 64..256 (256^2, 32 coils, 266 k entries:
-// 64 / 128 / 192 / 256 / 512 entries 172 / 110 / 91 / 87 / 111 us; 128^2, 1
-// coil, 44 k: 28 / 33 / 39 / 42 / 65), 3D 512..4096 (192^3, 16 coils, 20.6 M:
-// 2048 / 4096 / 8192 6.1 / 5.8 / 5.7 ms; the last one's longer partial sums
-// near the k-space centre round more).
-static int default_grid_chunk(const mrn_plan* P, int64_t E) {
-  if (P->ndim == 1) return 1024;
-  const int64_t lo = P->ndim == 2 ? 64 : 512, hi = P->ndim == 2 ? 256 : 4096;
-  const int64_t share = E / ((P->ndim == 2 ? 6 : 4) * (int64_t)P->sm_count);
-  return (int)std::min(hi, std::max(lo, share / 32 * 32));
+// Per slice {gridding entries, entries per work item} (chunk 0: grid_chunk_of).
+__global__ void k_slice_entries(const SliceGeom* __restrict__ sl, int ns, const int* __restrict__ off,
+                                const int* __restrict__ cnt, int64_t npts, int ndim, int sm_count, int chunk,
+                                int2* __restrict__ out) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= ns) return;
+  const int64_t p0 = sl[s].pt_off, p1 = p0 + sl[s].m;
+  int e = 0;
+  if (p1 > p0) e = (p1 < npts ? off[p1] : off[npts - 1] + cnt[npts - 1]) - off[p0];
+  out[s] = make_int2(e, chunk > 0 ? chunk : grid_chunk_of(ndim, sm_count, e));
 }
 
 static inline unsigned blocks_for(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
@@ -546,7 +564,7 @@ int mrn_plan_create(mrn_plan** out, int ndim, int n_slices, const int* im_size,
   // gridding tiles: 8x8 in 2D (one warp owns a tile), else the interpolation tile
   for (int i = 0; i < ndim; ++i) P->gtile[i] = (ndim >= 2 && !tile) ? 8 : P->tile[i];
   P->max_chunk = max_chunk > 0 ? max_chunk : (ndim == 2 ? 256 : 1024);
-  P->grid_chunk = max_chunk;  // 0: from the entry count, at mrn_plan_set_traj
+  P->grid_chunk = max_chunk;  // 0: from each slice's entry count, at mrn_plan_set_traj
 
   // Slices
   int64_t img = 0, ksp = 0, ugrid = 0, trjo = 0, pts = 0, xo = 0;
@@ -715,6 +733,7 @@ int mrn_plan_create(mrn_plan** out, int ndim, int n_slices, const int* im_size,
     P->cap_tiles = tmax;
   }
   PK(dev_alloc(&P->d_counts, 8));
+  PK(dev_alloc(&P->d_slice_ent, (size_t)n_slices));
   PK(dev_alloc(&P->d_sync, 64));
   CK(cudaMemset(P->d_sync, 0, 64 * sizeof(unsigned)));
   PK(dev_alloc(&P->d_red, (size_t)n_slices * kMaxRedBlocks));
@@ -825,7 +844,7 @@ int mrn_plan_destroy(mrn_plan* P) {
                   P->d_key_a, P->d_key_b, P->d_key_is, P->d_key_g, P->d_val_a, P->d_val_b, P->d_coord_tmp,
                   P->d_entry_cnt, P->d_tile_start_i, P->d_tile_end_i, P->d_tile_start_g,
                   P->d_tile_end_g, P->d_tile_nitems, P->d_tile_item_off, P->d_items_i,
-                  P->d_items_g, P->d_counts, P->d_split_tiles, P->d_cub_tmp, P->d_grid,
+                  P->d_items_g, P->d_counts, P->d_slice_ent, P->d_split_tiles, P->d_cub_tmp, P->d_grid,
                   P->d_ksp_tmp, P->d_sync, P->d_wmeta_i, P->d_wtab_i, P->d_wmeta_g,
                   P->d_wtab_g, P->d_part, P->d_items_tmp, P->d_sort_key[0], P->d_sort_key[1],
                   P->d_sort_idx[0], P->d_sort_idx[1], P->d_red, P->d_rowpart, P->d_rows, P->d_gather};
@@ -903,7 +922,10 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
   need = std::max(need, b);
   RK(ensure_cub(P, need));
 
-  int64_t E = 0;
+  // gridding entries, full work items, and bounds of the split tiles and their
+  // partial-tile slots, summed over the slices; the largest work item
+  int64_t E = 0, full = 0, max_split = 0, max_slots = 0;
+  int gchunk = 1;
   if (M > 0) {
     k_prep_points<<<blocks_for(M), 256, 0, st>>>(P->d_slices, P->nslices, ndim, P->kb, trj, M,
                                                   P->d_coord_tmp, P->d_key_a, P->d_val_a,
@@ -911,15 +933,26 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
     CK(cudaGetLastError());
     b = P->cub_tmp_bytes;
     CK(cub::DeviceScan::ExclusiveSum(P->d_cub_tmp, b, P->d_entry_cnt, eoff, (int)M, st));
-    k_total<<<1, 32, 0, st>>>(eoff, P->d_entry_cnt, M, P->d_counts + 2);
-    CK(cudaGetLastError());
-    int hE = 0;
-    CK(cudaMemcpyAsync(&hE, P->d_counts + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    E = hE;
   }
+  k_slice_entries<<<blocks_for(P->nslices), 256, 0, st>>>(P->d_slices, P->nslices, eoff, P->d_entry_cnt, M, ndim,
+                                                          P->sm_count, P->grid_chunk, P->d_slice_ent);
+  CK(cudaGetLastError());
+  if (M > 0) {
+    std::vector<int2> ent(P->nslices);
+    CK(cudaMemcpyAsync(ent.data(), P->d_slice_ent, ent.size() * sizeof(int2), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    for (const int2& e : ent) {
+      E += e.x;
+      full += e.x / e.y;
+      gchunk = std::max(gchunk, e.y);
+      if (e.x > e.y) {
+        max_split += e.x / e.y + 1;
+        max_slots += 2 * (int64_t)(e.x / e.y) + 1;
+      }
+    }
+  }
+  max_split = std::min<int64_t>(max_split, TG);
   P->n_entries_grid = E;
-  const int gchunk = P->grid_chunk > 0 ? P->grid_chunk : default_grid_chunk(P, E);
 
   // 2. gridding entry buffers grow on demand
   const int64_t capE = std::max<int64_t>(E, 1);
@@ -940,7 +973,7 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
       CK(cudaMemsetAsync(P->d_tile_end_g, 0, TG * sizeof(int), st));  // counts, until the ranges are built
       k_tile_hist<<<blocks_for(E), 256, 0, st>>>(P->d_key_b, E, P->d_tile_end_g);
       k_entry_codes<<<blocks_for(E), 256, 0, st>>>(P->d_slices, P->nslices, ndim, P->kb, P->d_coord_tmp, P->d_val_b,
-                                                   P->d_tile_end_g, gchunk, E, P->d_key_b);
+                                                   P->d_tile_end_g, P->d_slice_ent, E, P->d_key_b);
     }
     CK(cudaGetLastError());
     b = 0;
@@ -976,14 +1009,12 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
   // 5. work items, launched at capacities known from T, M and E alone, so the
   // host needs no further read-back: a tile with c entries makes
   // ceil(c / chunk) items (gridding: at least one), hence at most
-  // T + M / chunk + 1 of them; split gridding tiles have more than gchunk
-  // entries each (at most E / gchunk + 1 tiles) and ceil(c / gchunk) < 2 c / gchunk
-  // items each (fewer than 2 E / gchunk slots).
+  // T + M / chunk + 1 of them; split gridding tiles of a slice of e entries
+  // have more than its chunk entries each (at most e / chunk + 1 tiles) and
+  // ceil(c / chunk) < 2 c / chunk items each (fewer than 2 e / chunk + 2 slots).
   const int chunk = P->max_chunk;
   const int64_t max_items_i = M > 0 ? (int64_t)T + M / chunk + 1 : 0;
-  const int64_t max_items_g = (int64_t)TG + E / gchunk + 1;
-  const int64_t max_split = E > gchunk ? std::min<int64_t>(TG, E / gchunk + 1) : 0;
-  const int64_t max_slots = max_split > 0 ? 2 * (E / gchunk) + 1 : 0;
+  const int64_t max_items_g = (int64_t)TG + full + 1;
   if (max_items_i >= (int64_t)INT32_MAX || max_items_g >= (int64_t)INT32_MAX) return MRN_ERR_UNSUPPORTED;
   if (P->cap_items_i < max_items_i) {
     RK(dev_alloc(&P->d_items_i, (size_t)max_items_i));
@@ -1017,12 +1048,12 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
   // Emit into the staging list (padding pre-filled with slice = -1), then
   // order longest first: CTAs start in index order, so the last wave holds
   // short items instead of a few long tiles.
-  auto make_items = [&](int ntiles, int ch, int min_items, int64_t cap, int count_slot, int gridding,
+  auto make_items = [&](int ntiles, int ch, int64_t cap, int count_slot, int gridding,
                         const int* tstart, const int* tend, Item* out) -> int {
     if (cap == 0) return MRN_OK;
     CK(cudaMemsetAsync(P->d_items_tmp, 0xff, (size_t)cap * sizeof(Item), st));
-    k_item_counts<<<blocks_for(ntiles), 256, 0, st>>>(tstart, tend, ntiles, ch, min_items,
-                                                      P->d_tile_nitems);
+    k_item_counts<<<blocks_for(ntiles), 256, 0, st>>>(P->d_slices, P->nslices, P->d_slice_ent, tstart, tend, ntiles,
+                                                      ch, gridding, P->d_tile_nitems);
     size_t nb = P->cub_tmp_bytes;
     CK(cub::DeviceScan::ExclusiveSum(P->d_cub_tmp, nb, P->d_tile_nitems, P->d_tile_item_off, ntiles, st));
     k_emit_items<<<blocks_for(ntiles), 256, 0, st>>>(P->d_slices, P->nslices, tstart, tend,
@@ -1041,8 +1072,8 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
     CK(cudaGetLastError());
     return MRN_OK;
   };
-  RK(make_items(T, chunk, 0, max_items_i, 0, 0, P->d_tile_start_i, P->d_tile_end_i, P->d_items_i));
-  RK(make_items(TG, gchunk, 1, max_items_g, 1, 1, P->d_tile_start_g, P->d_tile_end_g, P->d_items_g));
+  RK(make_items(T, chunk, max_items_i, 0, 0, P->d_tile_start_i, P->d_tile_end_i, P->d_items_i));
+  RK(make_items(TG, gchunk, max_items_g, 1, 1, P->d_tile_start_g, P->d_tile_end_g, P->d_items_g));
   RK(build_wtabs(P, st));
   P->n_items_interp = max_items_i;
   P->n_items_grid = max_items_g;

@@ -88,3 +88,44 @@ def test_transforms_do_not_depend_on_the_other_slices(ims, coils):
         _, one_grid, one_back = transforms([ims[s]], [coils[s]], img[i].contiguous(), src[g].contiguous())
         assert torch.equal(grid[g], one_grid), f"forward, slice {s}"
         assert torch.equal(back[i], one_back), f"inverse, slice {s}"
+
+
+@pytest.mark.parametrize("ims,ms,coils,W", [
+    ([(48, 48), (203, 203), (64, 64), (160, 150), (56, 56)], [1600, 9000, 4800, 100000, 2000], [3, 4, 12, 20, 1], 6.0),
+    ([(48, 48), (64, 60), (90, 80)], [1600, 4800, 60000], [8, 8, 8], 4.5),
+    ([(24, 24, 24), (32, 28, 30), (24, 20, 16)], [6000, 500000, 3000], [2, 8, 5], 4.0),
+])
+def test_samples_and_grids_do_not_depend_on_the_other_slices(ims, ms, coils, W):
+    """Forward and adjoint of slices of very different sample counts, with a dense centre (split gridding tiles): the
+    bits of each slice in a plan of its own, at the default work-item sizes."""
+    from mr_recon_b200 import _lib
+    from mr_recon_b200.plan import Plan
+    rng = np.random.RandomState(len(ims) + coils[0])
+    d = len(ims[0])
+    trjs = []
+    for im, m in zip(ims, ms):
+        t = (rng.rand(m, d) - 0.5) * np.array(im)
+        t[::2] *= 0.3
+        trjs.append(t.astype(np.float32))
+    flat = lambda a: torch.from_numpy(np.concatenate([v.reshape(-1) for v in a])).to(DEV)  # noqa: E731
+
+    def run(ims, ms, coils, trj, img, ksp):
+        p = Plan(ims, ms, coils, 1.25, (W,) * d, device=DEV)
+        if d == 2:
+            p.set_option(_lib.MRN_OPT_GRID_LANES, 32)
+        p.set_traj(trj)
+        k, b = torch.empty_like(ksp), torch.empty_like(img)
+        p.forward(img, k)
+        p.adjoint(ksp, b)
+        return p, k, b
+
+    img = flat([_cplx(rng, (c, *im)) for im, c in zip(ims, coils)])
+    ksp = flat([_cplx(rng, (c, m)) for m, c in zip(ms, coils)])
+    both, k, b = run(ims, ms, coils, flat(trjs), img, ksp)
+    assert both.stats()["split_tiles"] > 0
+    for s in range(len(ims)):
+        i = slice(int(both.img_off[s]), int(both.img_off[s]) + coils[s] * int(np.prod(ims[s])))
+        q = slice(int(both.ksp_off[s]), int(both.ksp_off[s]) + coils[s] * ms[s])
+        _, k1, b1 = run([ims[s]], [ms[s]], [coils[s]], flat([trjs[s]]), img[i].contiguous(), ksp[q].contiguous())
+        assert torch.equal(k[q], k1), f"forward, slice {s}"
+        assert torch.equal(b[i], b1), f"adjoint, slice {s}"
