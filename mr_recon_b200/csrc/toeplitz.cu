@@ -62,6 +62,7 @@ struct ToepState {
     cufftHandle handle;
   };
   std::vector<Group> fft;
+  bool use_ffx = false;  // the plan's MRN_OPT_NATIVE_FFT when the state was built
   // native: the plan's slices on the padded grids
   bool native = false;
   std::vector<SliceGeom> hsl;
@@ -445,9 +446,9 @@ int mrn_plan_set_toeplitz(mrn_plan* P, const int* pad_size, const void* kern, vo
       // PadLast pads (np - n) / 2 on both sides: np - n must be even
       if (np < n || ((np - n) & 1)) return MRN_ERR_ARG;
     }
-  // same padded sizes as before: keep buffers and FFT plans, refresh the kernel
+  // same padded sizes and FFT option as before: keep buffers and FFT plans, refresh the kernel
   ToepState* T = toep(P);
-  bool same = T != nullptr;
+  bool same = T != nullptr && T->use_ffx == P->use_ffx;
   if (same)
     for (int s = 0; s < P->nslices && same; ++s)
       for (int i = 0; i < D; ++i) same &= T->h[s].np[i] == pad_size[s * D + i];
@@ -455,6 +456,7 @@ int mrn_plan_set_toeplitz(mrn_plan* P, const int* pad_size, const void* kern, vo
     toep_free(P);
     T = new ToepState();
     P->toep = T;
+    T->use_ffx = P->use_ffx;
     T->h.resize(P->nslices);
     int64_t goff = 0, koff = 0, prow = 0;
     for (int s = 0; s < P->nslices; ++s) {

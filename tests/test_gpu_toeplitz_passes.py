@@ -73,3 +73,24 @@ def test_toeplitz_passes(slices, coils):
         a, b = a + i.size, b + v.size
         assert np.linalg.norm(got - ref) <= 1e-6 * np.linalg.norm(ref)
         assert np.linalg.norm(sgot - sref) <= 1e-6 * np.linalg.norm(sref)
+
+
+def test_kernels_set_again_follow_the_fft_option():
+    """The same padded sizes after MRN_OPT_NATIVE_FFT changed: the bits of a plan that had the value from the start."""
+    from mr_recon_b200 import _lib
+    rng = np.random.default_rng(5)
+    kern = torch.from_numpy(cplx(rng, (96, 80))).to(DEV)
+    img = torch.from_numpy(cplx(rng, (3, 48, 40))).to(DEV)
+
+    def normal(plan, native):
+        plan.set_option(_lib.MRN_OPT_NATIVE_FFT, native)
+        plan.set_toeplitz(kern, [(96, 80)])
+        out = torch.empty_like(img)
+        plan.toeplitz_normal(img, out)
+        return out
+
+    make = lambda: Plan([(48, 40)], [0], [3], 1.25, (4.0, 4.0), device=DEV)  # noqa: E731
+    plan, fresh = make(), {n: normal(make(), n) for n in (0, 1)}
+    assert not torch.equal(fresh[0], fresh[1])
+    for native in (1, 0, 1):
+        assert torch.equal(normal(plan, native), fresh[native])
