@@ -249,9 +249,9 @@ int launch_turn(const FfxTurnSet& S, const FfxGrid& G, const float2* kern, cudaS
 // enough for either direction's padded first stage.
 static size_t turn_smem(const FfxTurn& t, int w) { return ((size_t)2 * t.fwd.n + (size_t)2 * t.buf * w) * sizeof(float2); }
 
-// One turning pass per slice (all slices native and direct: S.all of the set
-// built without chirp convolutions). kern_off: complex offset of a slice's
-// kernel, centred [n0][cells of the later axes].
+// One turning pass per slice of direct radices (g.native_fft; the others get an
+// empty one, whose blocks return). kern_off: complex offset of a slice's kernel,
+// centred [n0][cells of the later axes].
 int ffx_turn_build(FfxTurnSet& S, const FfxSet& F, int ndim, const std::vector<SliceGeom>& hsl,
                    const std::vector<int64_t>& kern_off, int sm_count) {
   S.release();
@@ -262,6 +262,10 @@ int ffx_turn_build(FfxTurnSet& S, const FfxSet& F, int ndim, const std::vector<S
   for (size_t s = 0; s < hsl.size(); ++s) {
     const SliceGeom& g = hsl[s];
     FfxTurn t{};
+    if (!g.native_fft) {
+      turns.push_back(t);
+      continue;
+    }
     for (const FfxTurn& o : turns)
       if (o.fwd.n == g.nos[0]) t = o;
     if (t.fwd.n == 0) {

@@ -94,3 +94,38 @@ def test_kernels_set_again_follow_the_fft_option():
     assert not torch.equal(fresh[0], fresh[1])
     for native in (1, 0, 1):
         assert torch.equal(normal(plan, native), fresh[native])
+
+
+@pytest.mark.parametrize("slices,coils", [
+    ([((24, 24), (48, 48)), ((46, 20), (92, 40)), ((30, 20), (60, 40)), ((46, 20), (92, 40))], [4, 3, 11, 9]),
+    ([((10, 12, 9), (20, 24, 23)), ((12, 10, 9), (24, 20, 27))], [5, 2]),
+])
+def test_normal_does_not_depend_on_the_other_slices(slices, coils):
+    """Padded sizes without direct radices (92, 23) beside others: each slice's normal, and its CG sum, has the bits
+    that it has in a plan of its own."""
+    rng = np.random.default_rng(len(slices))
+    ims, pads = [s[0] for s in slices], [s[1] for s in slices]
+    d = len(ims[0])
+    kerns = [cplx(rng, p) for p in pads]
+    imgs = [cplx(rng, (c, *im)) for c, im in zip(coils, ims)]
+    xs = [cplx(rng, im) for im in ims]
+    flat = lambda a: torch.from_numpy(np.concatenate([v.reshape(-1) for v in a])).to(DEV)  # noqa: E731
+
+    def run(sel):
+        pick = lambda a: [a[s] for s in sel]  # noqa: E731
+        plan = Plan(pick(ims), [0] * len(sel), pick(coils), 1.25, (4.0,) * d, device=DEV)
+        plan.set_toeplitz(flat(pick(kerns)), pick(pads))
+        img, x = flat(pick(imgs)), flat(pick(xs))
+        out, sense = torch.empty_like(img), torch.empty_like(x)
+        pap = torch.zeros(len(sel), dtype=torch.float64, device=DEV)
+        plan.toeplitz_normal(img, out)
+        plan.sense_normal_toeplitz(x, img, sense, 1.0, 0.5, pap)
+        return out, sense, pap
+
+    out, sense, pap = run(range(len(slices)))
+    a = b = 0
+    for s in range(len(slices)):
+        o1, s1, p1 = run([s])
+        assert torch.equal(out[a:a + o1.numel()], o1) and torch.equal(sense[b:b + s1.numel()], s1)
+        assert pap[s] == p1[0]
+        a, b = a + o1.numel(), b + s1.numel()
