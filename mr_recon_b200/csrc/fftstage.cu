@@ -253,6 +253,10 @@ int launch_pre(mrn_plan* P, PreMode mode, const float2* src, const float2* mps, 
   return e == cudaSuccess ? MRN_OK : cuda_fail(e);
 }
 
+// Threads that sum a row of nl pixels: from the slice's own row length (wider
+// slices of the plan may give the block more), as the order of its Re<xin, out>.
+__host__ __device__ constexpr int post_threads(int nl) { return nl <= 64 ? 64 : (nl <= 128 ? 128 : 256); }
+
 // SENSE post with one block per image row and one thread per pixel (the
 // per-warp row kernel above leaves a single 2D image on a few hundred warps):
 // out[q] = scale * apod(q) * sum_c conj(mps_c[q]) Y_c[(q - N//2) mod Nos]
@@ -297,7 +301,8 @@ k_post_sense(const SliceGeom* __restrict__ sl, int ns, const float* __restrict__
   float2* orow_p = out + g.x_off + orow * nl;
   const float2* xrow = xin ? xin + g.x_off + orow * nl : nullptr;
   double part = 0.0;
-  for (int j = threadIdx.x; j < nl; j += blockDim.x) {
+  const int nt = post_threads(nl);
+  for (int j = threadIdx.x; j < nl && (int)threadIdx.x < nt; j += nt) {
     int sj = j - h;
     if (sj < 0) sj += nosl;
     float ax = 0.f, ay = 0.f;
@@ -346,7 +351,7 @@ int launch_post_sense(mrn_plan* P, const SliceGeom* dsl, const float* apod, cons
   if (P->n_xrow <= 0) return MRN_OK;
   int nl = 1;
   for (const auto& g : P->h_slices) nl = std::max(nl, g.n[P->ndim - 1]);
-  const unsigned threads = nl <= 64 ? 64 : (nl <= 128 ? 128 : 256);
+  const unsigned threads = post_threads(nl);
   const unsigned rows = (unsigned)P->n_xrow;
   const int ns = P->nslices;
   if (P->ndim == 1)

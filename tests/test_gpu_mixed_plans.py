@@ -129,3 +129,32 @@ def test_samples_and_grids_do_not_depend_on_the_other_slices(ims, ms, coils, W):
         _, k1, b1 = run([ims[s]], [ms[s]], [coils[s]], flat([trjs[s]]), img[i].contiguous(), ksp[q].contiguous())
         assert torch.equal(k[q], k1), f"forward, slice {s}"
         assert torch.equal(b[i], b1), f"adjoint, slice {s}"
+
+
+def test_cg_sums_do_not_depend_on_the_other_slices():
+    """Re<x, A x> of rows of 40, 100 and 200 pixels in one plan and alone: the same float64 bits."""
+    from mr_recon_b200 import _lib
+    from mr_recon_b200.plan import Plan
+    rng = np.random.RandomState(3)
+    ims, coils, m = [(30, 40), (20, 100), (24, 200)], [2, 3, 8], 400
+    xs = [_cplx(rng, im) for im in ims]
+    mps = [_cplx(rng, (c, *im)) for c, im in zip(coils, ims)]
+    trjs = [((rng.rand(m, 2) - 0.5) * np.array(im)).astype(np.float32) for im in ims]
+    flat = lambda a: torch.from_numpy(np.concatenate([v.reshape(-1) for v in a])).to(DEV)  # noqa: E731
+
+    def sums(sel):
+        pick = lambda a: [a[s] for s in sel]  # noqa: E731
+        p = Plan(pick(ims), [m] * len(sel), pick(coils), 1.25, (6.0, 6.0), device=DEV)
+        p.set_option(_lib.MRN_OPT_GRID_LANES, 8)
+        p.set_traj(flat(pick(trjs)))
+        x = flat(pick(xs))
+        out, pap = torch.empty_like(x), torch.zeros(len(sel), dtype=torch.float64, device=DEV)
+        p.sense_normal(x, flat(pick(mps)), None, out, 1.0, 0.1, pap)
+        return out, pap
+
+    out, pap = sums([0, 1, 2])
+    at = 0
+    for s in range(3):
+        o1, p1 = sums([s])
+        assert torch.equal(out[at:at + o1.numel()], o1) and pap[s] == p1[0]
+        at += o1.numel()
