@@ -562,6 +562,8 @@ struct mrn_plan {
   // each block width, cut into CTAs of `chunk` sorted samples.
   struct GatherSet {
     int cb;        // coils per block of these slices
+    bool native;   // their plan grids are in coil blocks while MRN_OPT_NATIVE_FFT is on (else coil planes)
+    int max_coil;
     int nsl;       // slices
     int chunk;     // samples per CTA
     int nchunks;   // CTAs

@@ -1,7 +1,7 @@
 // Type-2 interpolation (grid -> samples) straight from a grid in coil blocks
 // ([coil block][cell][cb], grid_at): the default path of launch_interp for
-// 2D / 3D kernels of 5..8 candidate taps on grids the native FFT passes
-// transform, and for one-coil caller grids.
+// 2D / 3D kernels of 5..8 candidate taps, for the slices whose grids the native
+// FFT passes transform, and for one-coil caller grids.
 //
 // Reference: triton_interp/ungrid.py (_ungrid2d / _ungrid3d, :200-495). Tap
 // selection and weights are the reference's: taps j = lo + q, lo = ceil(u -
@@ -212,8 +212,8 @@ k_interp_gather(const int* __restrict__ slices, const int* __restrict__ first_ch
 constexpr int kTileWarps = 8;
 constexpr int kTileRun = 8;  // samples a warp takes at once
 
-// 2D, coil blocks of 8: a CTA per work item (interpolation tile) and group of
-// NB blocks. The tile and its halo come into shared memory as [cell][8 NB
+// 2D slices in coil blocks of 8: a CTA per work item (interpolation tile) and
+// group of NB blocks. The tile and its halo come into shared memory as [cell][8 NB
 // coils] by 16-byte asynchronous copies (a grid row of the region is
 // contiguous per block); a cell's row is padded by two coils, which keeps it
 // 16-byte aligned and puts the two samples a warp reads at once on any
@@ -236,7 +236,7 @@ k_interp_tile(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, 
   if (it.slice < 0) return;  // padding past the real items
   const SliceGeom& g = sl[it.slice];
   const int ncoil = g.ncoil, c0 = blockIdx.y * CW;
-  if (c0 >= ncoil) return;
+  if (c0 >= ncoil || g.cb != 8) return;  // slices of other blocks: k_interp_gather, k_interp_reg
   const int nc = min(CW, ncoil - c0);
   const int nos0 = g.nos[0], nos1 = g.nos[1];
   const int64_t gos = g.gos, m = g.m;
@@ -356,22 +356,25 @@ k_interp_tile(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, 
 
 // Slices by coil block, and the CTAs of each: chunks of kGatherChunk samples,
 // halved while they would leave SMs idle (never below one round of a
-// two-warp CTA).
+// two-warp CTA). Called with MRN_OPT_NATIVE_FFT at its default.
 int gather_setup(mrn_plan* P) {
   P->gather.clear();
   if (P->ndim < 2) return MRN_OK;
   std::vector<int> tab;
-  for (int cb : {1, 2, 4, 8}) {
+  for (int kind = 0; kind < 8; ++kind) {
     mrn_plan::GatherSet gs{};
-    gs.cb = cb;
+    const int cb = gs.cb = 1 << (kind & 3);
+    gs.native = kind < 4;
     gs.off = (int)tab.size();
     int64_t pts = 0;
-    for (int s = 0; s < P->nslices; ++s)
-      if (coil_block(P->h_slices[s].ncoil) == cb && P->h_slices[s].m > 0) {
-        tab.push_back(s);
-        pts += P->h_slices[s].m;
-        ++gs.nsl;
-      }
+    for (int s = 0; s < P->nslices; ++s) {
+      const SliceGeom& g = P->h_slices[s];
+      if (coil_block(g.ncoil) != cb || (g.native_fft != 0) != gs.native || g.m == 0) continue;
+      tab.push_back(s);
+      pts += g.m;
+      gs.max_coil = std::max(gs.max_coil, g.ncoil);
+      ++gs.nsl;
+    }
     if (gs.nsl == 0) continue;
     gs.chunk = kGatherChunk;
     while (gs.chunk > 2 * (32 / cb) && gs.chunk > 32 && pts / gs.chunk < 4 * (int64_t)P->sm_count) gs.chunk /= 2;
@@ -391,32 +394,43 @@ int gather_setup(mrn_plan* P) {
   return e == cudaSuccess ? MRN_OK : cuda_fail(e);
 }
 
-// Every slice's grid is in coil blocks: the plan grid when all FFT groups run
-// natively, a caller's grid (coil planes) when it has one coil.
-bool gather_ok(const mrn_plan* P, int layout) {
-  if (P->gather.empty() || P->coil_group_req > 0) return false;
-  if (layout == kInternal) return ffx_active(P) && P->ffx.all;
-  return P->max_coil == 1;
+// Slices of the plan grid that cuFFT transforms (coil planes, FFT order).
+static bool gather_rest(const mrn_plan* P) {
+  for (const auto& gs : P->gather)
+    if (!gs.native) return true;
+  return false;
 }
 
-// 2D plans whose slices all come in blocks of 8 coils and whose tile regions
-// fit: 256^2, 32 coils, 98,304 spiral samples, W 6: 60 us (68 with the
-// tile staged from coil planes) against 78 from global memory, whose 906 MB of
-// taps need more L1 than the CTAs of an SM have.
+// Some slices' grids are in coil blocks: plan grids of the native passes
+// (k_interp_reg takes the other slices), a caller's grid (coil planes) when it
+// has one coil.
+bool gather_ok(const mrn_plan* P, int layout) {
+  if (P->gather.empty() || P->coil_group_req > 0) return false;
+  if (layout != kInternal) return P->max_coil == 1;
+  return ffx_active(P) && P->gather[0].native && (!gather_rest(P) || interp_reg_ok(P));
+}
+
+// Each slice takes the kernel of its own grid. 2D, four slices of 12 to 32 coils,
+// 32 k samples each (76 us), with a fifth of 4 coils 90 us, where it sent all to
+// k_interp_gather 115; with a fifth that cuFFT transforms 117 to 120, where all
+// went to k_interp_reg 113 to 115 (its few CTAs run by themselves); 3D, 64^3 and
+// 96^3 with one of 56^3 that cuFFT transforms, 8 coils, 633 and 873.
+//
+// 2D slices in blocks of 8 coils whose tile regions fit: 256^2, 32 coils,
+// 98,304 spiral samples, W 6: 60 us (68 with the tile staged from coil planes)
+// against 78 from global memory, whose 906 MB of taps need more L1 than the
+// CTAs of an SM have.
 static size_t tile_smem(const mrn_plan* P, int nb) {
   const int K = P->kb.ntaps[0];
   return (size_t)(P->tmax_cells[0] + K - 1) * (P->tmax_cells[1] + K - 1) * (8 * nb + 2) * sizeof(float2);
 }
 
-int launch_interp_gather(mrn_plan* P, const float2* grid, int layout, float2* ksp, float scale, cudaStream_t st,
-                         RowIO rio) {
-  const int K = P->kb.ntaps[0];
-  if (P->ndim == 2 && layout == kInternal && P->gather.size() == 1 && P->gather[0].cb == 8) {
-    const int nb = P->max_coil <= 8 ? 1 : 2;
-    const size_t smem = tile_smem(P, nb);
-    if (smem <= 100 * 1024) {
-      const dim3 gd((unsigned)P->n_items_interp, (unsigned)((P->max_coil + 8 * nb - 1) / (8 * nb)));
-      int rc = MRN_OK;
+static int launch_tile(mrn_plan* P, int max_coil, const float2* grid, float2* ksp, float scale, cudaStream_t st,
+                       RowIO rio) {
+  const int K = P->kb.ntaps[0], nb = max_coil <= 8 ? 1 : 2;
+  const size_t smem = tile_smem(P, nb);
+  const dim3 gd((unsigned)P->n_items_interp, (unsigned)((max_coil + 8 * nb - 1) / (8 * nb)));
+  int rc = MRN_OK;
 #define MRN_TILE(KK, NN)                                                                                    \
   do {                                                                                                      \
     auto kern = k_interp_tile<KK, NN>;                                                                      \
@@ -426,18 +440,27 @@ int launch_interp_gather(mrn_plan* P, const float2* grid, int layout, float2* ks
                                               ksp, scale, rio);                                             \
   } while (0)
 #define MRN_TILE_N(KK) if (nb == 2) MRN_TILE(KK, 2); else MRN_TILE(KK, 1)
-      if (K == 5) { MRN_TILE_N(5); }
-      else if (K == 6) { MRN_TILE_N(6); }
-      else if (K == 7) { MRN_TILE_N(7); }
-      else { MRN_TILE_N(8); }
+  if (K == 5) { MRN_TILE_N(5); }
+  else if (K == 6) { MRN_TILE_N(6); }
+  else if (K == 7) { MRN_TILE_N(7); }
+  else { MRN_TILE_N(8); }
 #undef MRN_TILE_N
 #undef MRN_TILE
-      if (rc != MRN_OK) return rc;
-      cudaError_t e = cudaGetLastError();
-      return e == cudaSuccess ? MRN_OK : cuda_fail(e);
-    }
-  }
+  if (rc != MRN_OK) return rc;
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? MRN_OK : cuda_fail(e);
+}
+
+int launch_interp_gather(mrn_plan* P, const float2* grid, int layout, float2* ksp, float scale, cudaStream_t st,
+                         RowIO rio) {
+  const int K = P->kb.ntaps[0];
   for (const auto& gs : P->gather) {
+    if (layout == kInternal && !gs.native) continue;
+    if (P->ndim == 2 && layout == kInternal && gs.cb == 8 && tile_smem(P, gs.max_coil <= 8 ? 1 : 2) <= 100 * 1024) {
+      const int rc = launch_tile(P, gs.max_coil, grid, ksp, scale, st, rio);
+      if (rc != MRN_OK) return rc;
+      continue;
+    }
     const int* sl = P->d_gather + gs.off;
     const int sub = 32 / gs.cb;
     const int warps = std::max(2, std::min(kGatherWarps, gs.chunk / sub));
@@ -465,6 +488,8 @@ int launch_interp_gather(mrn_plan* P, const float2* grid, int layout, float2* ks
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e);
   }
+  if (layout == kInternal && gather_rest(P))
+    return launch_interp_reg(P, grid, layout, ksp, scale, nullptr, st, rio, true);
   return MRN_OK;
 }
 

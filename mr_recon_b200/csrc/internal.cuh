@@ -57,7 +57,8 @@ int launch_grid_warp(mrn_plan* P, const float2* ksp, const float* dcf, const flo
                      int layout, float2* grid, float scale, cudaStream_t st);
 bool interp_reg_ok(const mrn_plan* P);
 int launch_interp_reg(mrn_plan* P, const float2* grid, int layout, float2* ksp, float scale,
-                      const float2* temporal, cudaStream_t st, RowIO rio = RowIO{0, 0, nullptr});
+                      const float2* temporal, cudaStream_t st, RowIO rio = RowIO{0, 0, nullptr},
+                      bool skip_native = false);
 int launch_trajgrad_reg(mrn_plan* P, const float2* grid, int layout, const float2* samples, float* out,
                         float scale, cudaStream_t st);
 // Interpolation straight from a grid in coil blocks (gather.cu)

@@ -632,7 +632,7 @@ __global__ void __launch_bounds__(kRegInterpWarps * 32, (D == 3 && K > 5) ? 2 : 
 k_interp_reg(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KBParams kb,
              const float4* __restrict__ coord, const int* __restrict__ perm,
              const float2* __restrict__ grid, int layout, float2* __restrict__ ksp, float scale,
-             const float2* __restrict__ temporal, int cg, RowIO rio) {
+             const float2* __restrict__ temporal, int cg, RowIO rio, int skip_native) {
   constexpr int CW = 32 / SUB, CS = CW + 1, NW = kRegInterpWarps, NT = NW * 32;
   extern __shared__ float4 smem_f4[];
   float2* region = reinterpret_cast<float2*>(smem_f4);
@@ -644,7 +644,7 @@ k_interp_reg(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, K
   const SliceGeom* gp = sl + it.slice;
   const int ncoil = gp->ncoil;
   const int c0 = blockIdx.y * cg;
-  if (c0 >= ncoil) return;
+  if (c0 >= ncoil || (skip_native && gp->native_fft)) return;
   const int ncg = min(cg, ncoil - c0);
   int nos[3], hs[3], ext[3];
   const Frame f = frame_of(*gp, it.tile, D, false);
@@ -1027,7 +1027,7 @@ bool interp_reg_ok(const mrn_plan* P) {
 }
 
 int launch_interp_reg(mrn_plan* P, const float2* grid, int layout, float2* ksp, float scale,
-                      const float2* temporal, cudaStream_t st, RowIO rio) {
+                      const float2* temporal, cudaStream_t st, RowIO rio, bool skip_native) {
   if (P->n_items_interp == 0) return MRN_OK;
   int cg, ng;
   const int sub = interp_reg_sub(P, &cg, &ng);
@@ -1042,7 +1042,7 @@ int launch_interp_reg(mrn_plan* P, const float2* grid, int layout, float2* ksp, 
     if (rc == MRN_OK)                                                                               \
       kern<<<gdim, kRegInterpWarps * 32, smem, st>>>(P->d_items_i, P->d_slices, P->kb, P->d_coord_i, \
                                                      P->d_perm_i, grid, layout, ksp, scale, temporal, cg, \
-                                                     rio);                                            \
+                                                     rio, skip_native ? 1 : 0);                                            \
   } while (0)
 #define MRN_IREG_SUB(DD, KK)                     \
   if (sub == 4) MRN_IREG_LAUNCH(DD, KK, 4);      \

@@ -137,7 +137,7 @@ def test_cg_sums_do_not_depend_on_the_other_slices():
     from mr_recon_b200.plan import Plan
     rng = np.random.RandomState(3)
     ims, coils, m = [(30, 40), (20, 100), (24, 200)], [2, 3, 8], 400
-    xs = [_cplx(rng, im) for im in ims]
+    xs = [(_cplx(rng, im) * np.exp(rng.uniform(-9, 9, im))).astype(np.complex64) for im in ims]  # sums that round
     mps = [_cplx(rng, (c, *im)) for c, im in zip(coils, ims)]
     trjs = [((rng.rand(m, 2) - 0.5) * np.array(im)).astype(np.float32) for im in ims]
     flat = lambda a: torch.from_numpy(np.concatenate([v.reshape(-1) for v in a])).to(DEV)  # noqa: E731
