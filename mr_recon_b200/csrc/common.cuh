@@ -233,6 +233,8 @@ struct KBParams {
   float betad[kMaxDim];   // beta per dimension (sigpy-style per-axis kernel parameter)
   int uniform_beta;       // 1: every dimension uses beta (the fast kernels need this)
   int ntaps[kMaxDim];     // candidate taps floor(W_i) + 1
+  // candidate taps of the interpolation and gridding kernels that treat the last one as rare (window_taps)
+  int itaps, gtaps;
   float inv_radius[kMaxDim];  // 1 / (W_i / 2)
   int series;             // 1: coef holds the series below to float32 accuracy for this beta
   int nterms;             // terms the series needs for this beta: a multiple of 4 in [16, kKBTerms]

@@ -66,9 +66,9 @@ __device__ __forceinline__ float2 gather_fast(const float2* gp, int64_t sx, int6
   return acc;
 }
 
-// All K candidate taps with circular wrap: samples at the grid's edge, or with
-// a coordinate exactly W/2 from their last candidate tap. Out of line, so
-// its index arithmetic is not hoisted into every sample.
+// With circular wrap: samples at the grid's edge, or (whole widths, window_taps)
+// with a coordinate exactly W/2 from their K-th candidate tap, which the others
+// leave out. Out of line, so its index arithmetic is not hoisted into every sample.
 template <int D, int K, int CB>
 __device__ __noinline__ float2 gather_wrap(const float2* g, int64_t cell, int n0, int n1, int n2, const float* w) {
   float2 acc = make_float2(0.f, 0.f);
@@ -76,13 +76,15 @@ __device__ __noinline__ float2 gather_wrap(const float2* g, int64_t cell, int n0
   const int sl = (int)(cell % nl);
   const int64_t r = cell / nl;
   const int s1 = D == 3 ? (int)(r % n1) : 0, s0 = D == 3 ? (int)(r / n1) : (int)r;
+  const bool last = w[K - 1] != 0.f || w[8 + K - 1] != 0.f || (D == 3 && w[16 + K - 1] != 0.f);
+  const int ke = last ? K : K - 1;
 #pragma unroll 1
-  for (int a = 0; a < K; ++a) {
+  for (int a = 0; a < ke; ++a) {
     int x = s0 + a;
     if (x >= n0) x -= n0;
     float2 pa = make_float2(0.f, 0.f);
 #pragma unroll 1
-    for (int b = 0; b < (D == 3 ? K : 1); ++b) {
+    for (int b = 0; b < (D == 3 ? ke : 1); ++b) {
       int64_t row = x;
       if (D == 3) {
         int y = s1 + b;
@@ -93,6 +95,7 @@ __device__ __noinline__ float2 gather_wrap(const float2* g, int64_t cell, int n0
       float2 ra = make_float2(0.f, 0.f);
 #pragma unroll
       for (int c = 0; c < K; ++c) {
+        if (c == K - 1 && !last) break;
         int z = sl + c;
         if (z >= nl) z -= nl;
         const float v = w[8 * (D - 1) + c];
@@ -304,7 +307,7 @@ k_interp_tile(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, 
       const float* w = s_w[warp][j];
       const float2* rp = region + cell + coil;
       float2 acc = make_float2(0.f, 0.f);
-      // the K-th candidate of an axis has weight only when it lies exactly W/2 away
+      // the K-th tap of an axis has weight only when it lies exactly W/2 away (window_taps)
       const bool last = w[K - 1] != 0.f || w[8 + K - 1] != 0.f;
       float2 wl[K];
 #pragma unroll
@@ -421,13 +424,13 @@ bool gather_ok(const mrn_plan* P, int layout) {
 // against 78 from global memory, whose 906 MB of taps need more L1 than the
 // CTAs of an SM have.
 static size_t tile_smem(const mrn_plan* P, int nb) {
-  const int K = P->kb.ntaps[0];
+  const int K = P->kb.itaps;
   return (size_t)(P->tmax_cells[0] + K - 1) * (P->tmax_cells[1] + K - 1) * (8 * nb + 2) * sizeof(float2);
 }
 
 static int launch_tile(mrn_plan* P, int max_coil, const float2* grid, float2* ksp, float scale, cudaStream_t st,
                        RowIO rio) {
-  const int K = P->kb.ntaps[0], nb = max_coil <= 8 ? 1 : 2;
+  const int K = P->kb.itaps, nb = max_coil <= 8 ? 1 : 2;
   const size_t smem = tile_smem(P, nb);
   const dim3 gd((unsigned)P->n_items_interp, (unsigned)((max_coil + 8 * nb - 1) / (8 * nb)));
   int rc = MRN_OK;
@@ -453,7 +456,7 @@ static int launch_tile(mrn_plan* P, int max_coil, const float2* grid, float2* ks
 
 int launch_interp_gather(mrn_plan* P, const float2* grid, int layout, float2* ksp, float scale, cudaStream_t st,
                          RowIO rio) {
-  const int K = P->kb.ntaps[0];
+  const int K = P->kb.itaps;
   for (const auto& gs : P->gather) {
     if (layout == kInternal && !gs.native) continue;
     if (P->ndim == 2 && layout == kInternal && gs.cb == 8 && tile_smem(P, gs.max_coil <= 8 ? 1 : 2) <= 100 * 1024) {

@@ -68,6 +68,9 @@ int launch_interp_gather(mrn_plan* P, const float2* grid, int layout, float2* ks
                          RowIO rio = RowIO{0, 0, nullptr});
 // Register-tile gridding from sample-major rows (gridrows.cu)
 bool code_sort_ok(const mrn_plan* P);
+// Candidate taps K of the kernels whose fast form is K - 1 taps an axis
+// (k_interp_gather, k_interp_tile, k_grid_rows).
+void window_taps(mrn_plan* P);
 bool grid_rows_ok(const mrn_plan* P);
 int launch_rows(mrn_plan* P, const SliceGeom* slices, int ns, const float2* ksp, const float* dcf, float2* rows,
                 cudaStream_t st);

@@ -130,10 +130,10 @@ __global__ void k_prep_points(const SliceGeom* __restrict__ sl, int ns, int ndim
 }
 
 // Start of a gridding entry's window of K - 1 cells along the last axis (tile
-// `tile` of it), or 10 - K where all K candidate taps lie inside the tile: the
+// `tile` of it; K: gtaps), or 10 - K where all K taps lie inside the tile: the
 // order of the register-tile gridding's entries within a tile.
 __device__ __forceinline__ int window_code(const SliceGeom& g, const KBParams& kb, float u, int tile, int i) {
-  const int K = kb.ntaps[i], KW = K - 1, n = g.nos[i], org = tile_begin(tile, n, g.gntile[i]);
+  const int K = kb.gtaps, KW = K - 1, n = g.nos[i], org = tile_begin(tile, n, g.gntile[i]);
   const int size = tile_begin(tile + 1, n, g.gntile[i]) - org;
   const int lo = (int)ceilf(__fsub_rn(u, kb.radius[i]));
   int st = (lo < 0 ? lo + n : (lo >= n ? lo - n : lo)) - org;
@@ -908,6 +908,7 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
   const int gbits = bits + code_bits;
   P->traj_set = false;
   P->code_sorted = code_bits > 0;
+  window_taps(P);
 
   // 1. coordinates, interpolation keys, gridding entry counts
   int* eoff = P->d_entry_cnt + std::max<int64_t>(M, 1);

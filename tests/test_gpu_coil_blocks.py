@@ -186,3 +186,34 @@ def test_wide_transforms(nos, C):
     # one rounding of the coil product (and of the sum of up to 33 coils) apart
     assert _rel(ks.cpu().numpy(), kp.cpu().numpy()) < 1e-6
     assert _rel(xs.cpu().numpy(), (mps.conj() * back).sum(0).cpu().numpy()) < 1e-6
+
+
+@pytest.mark.parametrize("W", [4.5, 5.25, 6.5])
+@pytest.mark.parametrize("im,C", [((48, 40), 1), ((48, 40), 4), ((64, 45), 9), ((12, 10), 3), ((24, 20, 28), 2), ((24, 20, 28), 9),
+                                  ((13, 24, 24), 5)])
+def test_widths_that_are_not_whole(im, C, W):
+    """Half of the footprints of an axis have floor(W) taps there and half one more: forward, and adjoint with split
+    tiles, with samples on grid points and at the seam, on grids with room for one more tap and without."""
+    from mr_recon_b200.fourier import b200_nufft
+    from mr_recon_b200 import _lib
+    d, M = len(im), 900
+    rng = np.random.RandomState(C + int(8 * W))
+    trj = ((rng.rand(1, M, d) - 0.5) * np.array(im) * 1.2).astype(np.float32)
+    trj[:, ::7] = np.round(trj[:, ::7])
+    trj[:, 1::3] *= 0.2
+    trj[:, 2::11] = -np.array(im) / 2.0
+    img = (rng.randn(1, C, *im) + 1j * rng.randn(1, C, *im)).astype(np.complex64)
+    ksp = (rng.randn(1, C, M) + 1j * rng.randn(1, C, M)).astype(np.complex64)
+    nf = b200_nufft(im, oversamp=1.25, width=W)
+    on = O.KBNufftOracle(im, 1.25, W)
+    t = torch.from_numpy(trj).to(DEV)
+    # the tolerance of the repository's parity tests (float32 weights and sums)
+    assert _rel(nf.forward(torch.from_numpy(img).to(DEV), t).cpu().numpy(), on.forward(img, trj)) < 1e-5
+    assert _rel(nf.adjoint(torch.from_numpy(ksp).to(DEV), t).cpu().numpy(), on.adjoint(ksp, trj)) < 1e-5
+    from mr_recon_b200.plan import Plan
+    p = Plan([im], [M], [C], 1.25, (W,) * d, device=DEV)
+    p.set_option(_lib.MRN_OPT_GRID_CHUNK, 40)
+    p.set_traj(t.reshape(-1))
+    back = torch.empty(p.n_img, dtype=torch.complex64, device=DEV)
+    p.adjoint(torch.from_numpy(ksp).to(DEV), back)
+    assert _rel(back.cpu().numpy().reshape(img.shape), on.adjoint(ksp, trj)) < 1e-5
