@@ -354,6 +354,64 @@ k_grid_rows(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KB
   }
   cp_async_wait<0>();
 
+  // A sample that is not finite times a weight of zero (rows and planes of the
+  // tile outside its footprint, the ends of its window) spoils cells it does
+  // not belong to. Such a sum never becomes finite again, so the tile's sums
+  // tell (one product a cell); the tile is then added up once more, only where
+  // there is weight.
+  float2 zero = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < T; ++b) zero = __ffma2_rn(acc[a][b], make_float2(0.f, 0.f), zero);
+  const bool bad = coil < ncg && !(zero.x == 0.f && zero.y == 0.f);
+  if (NWARP == 1 ? __any_sync(0xffffffffu, bad) : __syncthreads_or(bad)) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < T; ++b) acc[a][b] = make_float2(0.f, 0.f);
+#pragma unroll 1
+    for (int bi = 0; bi < nbatch; ++bi) {
+      sync();  // the batch before is read
+      copy_coords(bi);
+      cp_async_commit();
+      cp_async_wait<0>();
+      sync();
+      copy_values(bi);
+      cp_async_commit();
+      weights(bi);
+      cp_async_wait<0>();
+      sync();
+      const int b2 = bi & 1, nb = batch_len(bi);
+#pragma unroll 1
+      for (int j = stream; j < nb; j += grid_streams<D, CW>()) {
+        const GEntry<D, CW>& e = s.e[b2][j];
+        const int zc = (int)(s.code[b2][j] & 0xffu), z0 = zc == NW ? 0 : zc, nz = zc == NW ? T : KW;
+        float2 v = e.v[coil];
+        if (TEMP) {
+          const float2 t = s.t[b2][j];
+          v = make_float2(v.x * t.x + v.y * t.y, v.y * t.x - v.x * t.y);
+        }
+        if (D == 3) {
+          const float w = e.wx[plane];
+          if (w == 0.f) continue;
+          v = __fmul2_rn(make_float2(w, w), v);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float w = e.wy[4 * half + r];
+          const float2 v2 = __fmul2_rn(make_float2(w, w), v);
+#pragma unroll
+          for (int z = 0; z < T; ++z) {
+            const int c = z - z0;
+            const float2 wz = c >= 0 && c < nz ? e.wz[c] : make_float2(0.f, 0.f);
+            if (w != 0.f && wz.x != 0.f) acc[r][z] = __ffma2_rn(wz, v2, acc[r][z]);
+          }
+        }
+      }
+    }
+  }
+
   if (grid_streams<D, CW>() > 1) {  // add the streams' tiles
 #pragma unroll
     for (int a = 0; a < 4; ++a)
@@ -492,7 +550,7 @@ bool code_sort_ok(const mrn_plan* P) {
 // of an axis have all candidates, so there the kernels count one more, which
 // never has weight. Interpolation, up to W 7 (8 taps a row): 3D, 96^3, 8 coils,
 // 1 M samples, W 4.5 / 5.5 / 6.5: 830 / 1510 / 1780 -> 510 / 759 / 1138 us. Gridding
-// in 2D up to W 6: 4 coils, 98,304 samples, W 4.5 / 5.5: 59 / 64 -> 54 / 58 us (3D, where
+// in 2D up to W 6: 4 coils, 98,304 samples, W 4.5 / 5.5: 59 / 64 -> 56 / 59 us (3D, where
 // every window costs four rows of a plane: W 4.5 / 5.5 / 6.5 648 / 893 / 1252 -> 642 / 930
 // / 1413, so not there).
 // Neither where a grid or a gridding tile is too small.

@@ -217,3 +217,41 @@ def test_widths_that_are_not_whole(im, C, W):
     back = torch.empty(p.n_img, dtype=torch.complex64, device=DEV)
     p.adjoint(torch.from_numpy(ksp).to(DEV), back)
     assert _rel(back.cpu().numpy().reshape(img.shape), on.adjoint(ksp, trj)) < 1e-5
+
+
+@pytest.mark.parametrize("im,os_,W,C", [((40, 32), 1.25, 6, 1), ((40, 32), 1.25, 4, 3), ((48, 40), 1.25, 4.5, 12), ((40, 32), 2.0, 7, 35),
+                                        ((16, 12, 20), 1.25, 4, 1), ((16, 20, 12), 1.5, 6, 3), ((12, 16, 16), 2.0, 5, 12),
+                                        ((16, 12, 20), 1.25, 4, 19)])
+@pytest.mark.parametrize("chunk", [40, 100000])
+def test_samples_that_are_not_finite_stay_in_their_footprints(im, os_, W, C, chunk):
+    """Gridding with infinite and NaN samples of some coils: exactly the cells with weight of theirs are not finite,
+    and the others are what they are with those samples zero."""
+    from mr_recon_b200 import _lib
+    from mr_recon_b200.plan import Plan
+    d, M = len(im), 500
+    rng = np.random.RandomState(C + int(W))
+    trj = ((rng.rand(M, d) - 0.5) * np.array(im) * 1.1).astype(np.float32)
+    trj[::2] *= 0.3
+    trj[::9] = np.round(trj[::9])
+    p = Plan([im], [M], [C], os_, (W,) * d, device=DEV)
+    p.set_option(_lib.MRN_OPT_GRID_CHUNK, chunk)
+    p.set_traj(torch.from_numpy(trj).to(DEV).reshape(-1))
+    shape = (C, *p.os_sizes[0])
+
+    def grid(k):
+        g = torch.empty(shape, dtype=torch.complex64, device=DEV)
+        p.grid(k, g, 0.5)
+        return g
+
+    ksp = torch.from_numpy((rng.randn(C, M) + 1j * rng.randn(C, M)).astype(np.complex64)).to(DEV)
+    where = torch.zeros((C, M), dtype=torch.bool, device=DEV)
+    for c, m, v in [(0, 3, complex("inf")), (C - 1, 9, complex("nan")), (C // 2, 18, complex(0, float("-inf")))]:
+        ksp[c, m] = v
+        where[c, m] = True
+    got = grid(ksp)
+    bad = ~(torch.isfinite(got.real) & torch.isfinite(got.imag))
+    assert torch.equal(bad, grid(where.to(torch.complex64)) != 0)
+    want = grid(torch.where(where, torch.zeros_like(ksp), ksp))
+    got, want = got[~bad].cpu().numpy(), want[~bad].cpu().numpy()
+    # the same terms in another order: a few ulp of float32 sums of up to a few hundred
+    assert _rel(got, want) < 1e-6
