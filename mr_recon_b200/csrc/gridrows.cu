@@ -337,15 +337,16 @@ k_grid_rows(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KB
       bool meet = h32 + lane < nb;
       if (D == 3) meet &= ((mine >> (8 + (warp % NPG) * PPW)) & ((1u << PPW) - 1u)) != 0u;
       if (D == 3 || CW == 32) meet &= ((mine >> (16 + 4 * half)) & 15u) != 0u;
-      // windows in the order of all 32 entries, also those the warp skips: a
-      // cell's order does not depend on which planes share its warp (CW)
+      // 3D: windows in the order of all 32 entries, also those the warp skips, so
+      // that a cell's order does not depend on which planes share its warp (CW;
+      // in 2D MRN_OPT_GRID_LANES fixes it)
       unsigned act = __ballot_sync(0xffffffffu, meet), left = 0xffffffffu;
       while (act) {
-        const int code = __shfl_sync(0xffffffffu, zcode, __ffs(left) - 1);
+        const int code = __shfl_sync(0xffffffffu, zcode, __ffs(D == 3 ? left : act) - 1);
         unsigned same = __ballot_sync(0xffffffffu, zcode == code);
-        left &= ~same;
+        if (D == 3) left &= ~same;
         same &= act;
-        if (!same) continue;
+        if (D == 3 && !same) continue;
         act &= ~same;
         RunBody<D, CW, B, TEMP> body{acc, s, b2, h32, plane, half, coil, stream, same};
         body.template dispatch<KW>(code);
@@ -358,7 +359,9 @@ k_grid_rows(const Item* __restrict__ items, const SliceGeom* __restrict__ sl, KB
   // tile outside its footprint, the ends of its window) spoils cells it does
   // not belong to. Such a sum never becomes finite again, so the tile's sums
   // tell (one product a cell); the tile is then added up once more, only where
-  // there is weight.
+  // there is weight. Costs 3 us of 101 at 256^2, 32 coils and 0.04 ms of 5.8 at
+  // 192^3, 16 coils, for the loop's schedule more than for the products (out of
+  // line 0 us, but 0.2 ms in 3D, which spills).
   float2 zero = make_float2(0.f, 0.f);
 #pragma unroll
   for (int a = 0; a < 4; ++a)
