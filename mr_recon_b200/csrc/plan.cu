@@ -81,20 +81,19 @@ __device__ __forceinline__ int find_slice_by_tile(const SliceGeom* sl, int ns, i
 
 // Distinct tiles of one dimension touched by the valid taps of a sample at
 // wrapped coordinate u: taps j = lo + q, valid iff |(float)j - u| <= r (the
-// float32 mask of weights1d..3d, kernels.py:268-393), cell = j mod nos.
-__device__ __forceinline__ int dim_tiles(float u, float r, int ntaps, int nos, int nt,
-                                         int* tiles) {
+// float32 mask of weights1d..3d, kernels.py:268-393), cell = j mod nos. The valid
+// taps are a run and tiles have at least ntaps - 1 cells (tiles_for), so they
+// are those of its ends.
+__device__ __forceinline__ int dim_tiles(float u, float r, int ntaps, int nos, int nt, int (&tiles)[2]) {
   const int lo = (int)ceilf(__fsub_rn(u, r));
-  int n = 0;
-  for (int q = 0; q < ntaps; ++q) {
-    const float dx = __fsub_rn((float)(lo + q), u);
-    if (!(fabsf(dx) <= r)) continue;
-    const int t = nt == 1 ? 0 : tile_of(pos_mod(lo + q, nos), nos, nt);
-    bool seen = false;
-    for (int z = 0; z < n; ++z) seen |= (tiles[z] == t);
-    if (!seen) tiles[n++] = t;
-  }
-  return n;
+  auto valid = [&](int q) { return fabsf(__fsub_rn((float)(lo + q), u)) <= r; };
+  int q0 = 0, q1 = ntaps - 1;
+  while (q0 <= q1 && !valid(q0)) ++q0;
+  while (q1 > q0 && !valid(q1)) --q1;
+  if (q0 > q1) return 0;
+  tiles[0] = nt == 1 ? 0 : tile_of(pos_mod(lo + q0, nos), nos, nt);
+  tiles[1] = nt == 1 ? 0 : tile_of(pos_mod(lo + q1, nos), nos, nt);
+  return tiles[0] == tiles[1] ? 1 : 2;
 }
 
 // Per sample: scaled, wrapped coordinates (fourier.py:420-430 then
@@ -120,7 +119,7 @@ __global__ void k_prep_points(const SliceGeom* __restrict__ sl, int ns, int ndim
     const int lo = (int)ceilf(__fsub_rn(v, kb.radius[i]));
     const int t0 = tile_of(pos_mod(lo, g.nos[i]), g.nos[i], g.ntile[i]);
     lin = lin * g.ntile[i] + t0;
-    int tiles[kMaxTaps];
+    int tiles[2];
     ntouch *= dim_tiles(v, kb.radius[i], kb.ntaps[i], g.nos[i], g.gntile[i], tiles);
   }
   coord[p] = make_float4(u[0], u[1], u[2], 0.f);
@@ -142,10 +141,11 @@ __device__ __forceinline__ int window_code(const SliceGeom& g, const KBParams& k
   return last && st >= 0 && st + K <= size ? 10 - K : min(max(st, 0), size - KW);
 }
 
-// Emit (tile, point) gridding entries at the scanned offsets.
+// Emit (tile, point) gridding entries at the scanned offsets; with code_bits
+// the key is the tile above kGPartBits zeros and the window code.
 __global__ void k_emit_entries(const SliceGeom* __restrict__ sl, int ns, int ndim, KBParams kb,
                                const float4* __restrict__ coord, int64_t npts,
-                               const int* __restrict__ eoff, unsigned* __restrict__ key,
+                               const int* __restrict__ eoff, int code_bits, unsigned* __restrict__ key,
                                int* __restrict__ val) {
   int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= npts) return;
@@ -153,10 +153,13 @@ __global__ void k_emit_entries(const SliceGeom* __restrict__ sl, int ns, int ndi
   const SliceGeom& g = sl[s];
   const float4 c4 = coord[p];
   const float uu[3] = {c4.x, c4.y, c4.z};
-  int tiles[kMaxDim][kMaxTaps];
+  int tiles[kMaxDim][2] = {};
   int nt[kMaxDim] = {1, 1, 1};
   for (int i = 0; i < ndim; ++i)
     nt[i] = dim_tiles(uu[i], kb.radius[i], kb.ntaps[i], g.nos[i], g.gntile[i], tiles[i]);
+  unsigned win[2] = {0u, 0u};
+  for (int c = 0; code_bits > 0 && c < nt[ndim - 1]; ++c)
+    win[c] = (unsigned)window_code(g, kb, uu[ndim - 1], tiles[ndim - 1][c], ndim - 1);
   int o = eoff[p];
   for (int a = 0; a < nt[0]; ++a)
     for (int b = 0; b < (ndim > 1 ? nt[1] : 1); ++b)
@@ -164,37 +167,33 @@ __global__ void k_emit_entries(const SliceGeom* __restrict__ sl, int ns, int ndi
         int lin = tiles[0][a];
         if (ndim > 1) lin = lin * g.gntile[1] + tiles[1][b];
         if (ndim > 2) lin = lin * g.gntile[2] + tiles[2][c];
-        key[o] = (unsigned)(g.gtile_base + lin);
+        const int w = ndim == 3 ? c : b;
+        key[o] = (unsigned)(g.gtile_base + lin) << code_bits | (w == 0 ? win[0] : win[1]);
         val[o] = (int)p;
         ++o;
       }
 }
 
-// Entries per tile.
-__global__ void k_tile_hist(const unsigned* __restrict__ key, int64_t n, int* __restrict__ cnt) {
+// Entries per tile (192^3 kooshball, 20.6 M entries: 242 us, one atomic per entry 535).
+__global__ void k_tile_hist(const unsigned* __restrict__ key, int code_bits, int64_t n, int* __restrict__ cnt) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
-  const unsigned k = key[e];
+  const unsigned k = key[e] >> code_bits;
   const unsigned peers = __match_any_sync(__activemask(), k);
   if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(cnt + k, __popc(peers));
 }
 
-// Append the window code and, in tiles of more entries than a work item of
-// their slice takes, the part of the trajectory to the tile keys.
-__global__ void k_entry_codes(const SliceGeom* __restrict__ sl, int ns, int ndim, KBParams kb,
-                              const float4* __restrict__ coord, const int* __restrict__ val,
+// Put the part of the trajectory into the keys of tiles of more entries than a
+// work item of their slice takes.
+__global__ void k_entry_parts(const SliceGeom* __restrict__ sl, int ns, const int* __restrict__ val,
                               const int* __restrict__ cnt, const int2* __restrict__ ent, int64_t n,
                               unsigned* __restrict__ key) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
-  const int t = (int)key[e], p = val[e];
-  const int s = find_slice_by_tile(sl, ns, t, 1);
+  const int t = (int)(key[e] >> kGCodeBits), s = find_slice_by_tile(sl, ns, t, 1);
+  if (cnt[t] <= ent[s].y) return;
   const SliceGeom& g = sl[s];
-  const int i = ndim - 1;
-  const float4 c4 = coord[p];
-  const unsigned code = (unsigned)window_code(g, kb, i == 2 ? c4.z : c4.y, (t - g.gtile_base) % g.gntile[i], i);
-  const unsigned part = cnt[t] > ent[s].y ? (unsigned)(((int64_t)p - g.pt_off) * (1 << kGPartBits) / g.m) : 0u;
-  key[e] = (unsigned)t << kGCodeBits | part << kGWinBits | code;
+  key[e] |= (unsigned)(((int64_t)val[e] - g.pt_off) * (1 << kGPartBits) / g.m) << kGWinBits;
 }
 
 __global__ void k_gather_coords(const float4* __restrict__ src, const int* __restrict__ perm,
@@ -902,10 +901,14 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
   const int TT = std::max(T, TG);
   if (P->cap_tiles < TT) return MRN_ERR_STATE;  // a failed retile left the tile arrays short
   const int ndim = P->ndim;
-  int bits = 1;
-  while (bits < 31 && (1ll << bits) <= (long long)TT) ++bits;
-  const int code_bits = code_sort_ok(P) && bits + kGCodeBits <= 31 ? kGCodeBits : 0;
-  const int gbits = bits + code_bits;
+  auto bits_of = [](int n) {
+    int bits = 1;
+    while (bits < 31 && (1ll << bits) <= (long long)n) ++bits;
+    return bits;
+  };
+  const int bits = bits_of(T);
+  const int code_bits = code_sort_ok(P) && bits_of(TG) + kGCodeBits <= 31 ? kGCodeBits : 0;
+  const int gbits = bits_of(TG) + code_bits;
   P->traj_set = false;
   P->code_sorted = code_bits > 0;
   window_taps(P);
@@ -969,12 +972,12 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
   // 3. emit gridding entries and sort both lists by tile (stable)
   if (M > 0) {
     k_emit_entries<<<blocks_for(M), 256, 0, st>>>(P->d_slices, P->nslices, ndim, P->kb,
-                                                   P->d_coord_tmp, M, eoff, P->d_key_b, P->d_val_b);
+                                                   P->d_coord_tmp, M, eoff, code_bits, P->d_key_b, P->d_val_b);
     if (code_bits > 0 && E > 0) {
       CK(cudaMemsetAsync(P->d_tile_end_g, 0, TG * sizeof(int), st));  // counts, until the ranges are built
-      k_tile_hist<<<blocks_for(E), 256, 0, st>>>(P->d_key_b, E, P->d_tile_end_g);
-      k_entry_codes<<<blocks_for(E), 256, 0, st>>>(P->d_slices, P->nslices, ndim, P->kb, P->d_coord_tmp, P->d_val_b,
-                                                   P->d_tile_end_g, P->d_slice_ent, E, P->d_key_b);
+      k_tile_hist<<<blocks_for(E), 256, 0, st>>>(P->d_key_b, code_bits, E, P->d_tile_end_g);
+      k_entry_parts<<<blocks_for(E), 256, 0, st>>>(P->d_slices, P->nslices, P->d_val_b, P->d_tile_end_g, P->d_slice_ent, E,
+                                                   P->d_key_b);
     }
     CK(cudaGetLastError());
     b = 0;
