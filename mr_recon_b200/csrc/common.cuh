@@ -471,6 +471,7 @@ struct mrn_plan {
   std::vector<mrn::SliceGeom> h_slices;
   int64_t n_img = 0, n_ksp = 0, n_grid = 0, n_trj = 0, n_pts = 0, n_x = 0;
   int64_t n_igrid = 0;  // elements of d_grid (place_grids, ffx.cu)
+  bool tight_grid = false;  // no room for partly filled coil blocks
   int64_t n_prow = 0, n_irow = 0, n_xrow = 0;  // row counts of the grid / image layouts
   int ntiles = 0;   // interpolation tiles, all slices
   int ngtiles = 0;  // gridding tiles, all slices

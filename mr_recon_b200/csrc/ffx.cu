@@ -255,7 +255,7 @@ bool ffx_pays(int ndim, const int* nos, int ncoil) {
 
 // Build the native FFT of a grid buffer: per native group its axes' plans and
 // tables, and per axis the lists of slices that run together. The slices of a
-// group have one grid and one image size.
+// group have one grid and one image size, and `cb` coils a block of their grids.
 int ffx_build(FfxSet& S, int ndim, const std::vector<SliceGeom>& hsl, const std::vector<FfxGroupSpec>& spec,
               int sm_count) {
   S.release();
@@ -324,7 +324,7 @@ int ffx_build(FfxSet& S, int ndim, const std::vector<SliceGeom>& hsl, const std:
           bool used = false;
           ps.narrow = narrow;
           for (int s : fg.slices) {
-            const int cb = coil_block(hsl[s].ncoil);
+            const int cb = hsl[s].cb;
             if ((a == D - 1 && cb < 8) != (narrow != 0)) continue;
             used = true;
             list.push_back(FfxSlice{s, (int)passes.size()});
@@ -382,6 +382,14 @@ int ffx_inv(const FfxSet& S, const FfxGrid& G, float2* out, float scale, cudaStr
 
 bool ffx_active(const mrn_plan* P) { return P->ffx.ok && P->use_ffx; }
 
+// Coils per block of a slice's native grid: coil_block, or (no room for partly
+// filled blocks) the widest that the coils fill.
+static int native_block(const mrn_plan* P, int ncoil) {
+  int cb = coil_block(ncoil);
+  while (P->tight_grid && ncoil % cb != 0) cb /= 2;
+  return cb;
+}
+
 // Lay the slices' grids out in d_grid, group by group: native groups in coil
 // blocks, centred, each slice from a multiple of 8 elements on (the
 // interpolation copies 16 bytes at a time, and the grids before it may have
@@ -397,7 +405,7 @@ static int64_t place_grids(mrn_plan* P, bool use_native) {
     for (int s : fg.slices) {
       SliceGeom& g = P->h_slices[s];
       g.native_fft = native ? 1 : 0;
-      g.cb = native ? coil_block(g.ncoil) : 1;
+      g.cb = native ? native_block(P, g.ncoil) : 1;
       for (int i = 0; i < P->ndim; ++i) g.hshift[i] = native ? 0 : g.nos[i] / 2;
       if (native) off = (off + 7) / 8 * 8;
       g.grid_off = off;
@@ -417,6 +425,7 @@ int ffx_refresh(mrn_plan* P) {
 int ffx_setup(mrn_plan* P) {
   P->ffx.release();
   if (P->flags & MRN_PLAN_RAW) return MRN_OK;
+  for (SliceGeom& g : P->h_slices) g.cb = native_block(P, g.ncoil);
   std::vector<FfxGroupSpec> spec;
   for (const auto& f : P->fft) spec.push_back(FfxGroupSpec{f.native, f.slices});
   const int rc = ffx_build(P->ffx, P->ndim, P->h_slices, spec, P->sm_count);

@@ -372,7 +372,7 @@ int gather_setup(mrn_plan* P) {
     int64_t pts = 0;
     for (int s = 0; s < P->nslices; ++s) {
       const SliceGeom& g = P->h_slices[s];
-      if (coil_block(g.ncoil) != cb || (g.native_fft != 0) != gs.native || g.m == 0) continue;
+      if (g.cb != cb || (g.native_fft != 0) != gs.native || g.m == 0) continue;
       tab.push_back(s);
       pts += g.m;
       gs.max_coil = std::max(gs.max_coil, g.ncoil);

@@ -463,6 +463,7 @@ static int ensure_cub(mrn_plan* P, size_t bytes) {
   if (bytes <= P->cub_tmp_bytes && P->d_cub_tmp) return MRN_OK;
   if (P->d_cub_tmp) cudaFree(P->d_cub_tmp);
   P->d_cub_tmp = nullptr;
+  P->cub_tmp_bytes = 0;
   cudaError_t e = cudaMalloc(&P->d_cub_tmp, bytes);
   if (e != cudaSuccess) return cuda_fail(e);
   P->cub_tmp_bytes = bytes;
@@ -739,7 +740,14 @@ int mrn_plan_create(mrn_plan** out, int ndim, int n_slices, const int* im_size,
   PK(dev_alloc(&P->d_rowpart, (size_t)std::max<int64_t>(P->n_xrow, 1)));
   if (!raw) {
     PK(ffx_setup(P));
-    PK(dev_alloc(&P->d_grid, std::max<int64_t>(P->n_igrid, 1)));
+    if (dev_alloc(&P->d_grid, std::max<int64_t>(P->n_igrid, 1)) != MRN_OK) {
+      // without room for whole coil blocks: blocks that the coils fill
+      cudaGetLastError();
+      P->d_grid = nullptr;
+      P->tight_grid = true;
+      PK(ffx_setup(P));
+      PK(dev_alloc(&P->d_grid, std::max<int64_t>(P->n_igrid, 1)));
+    }
     PK(dev_alloc(&P->d_ksp_tmp, std::max<int64_t>(P->n_ksp, 1)));
     PK(cufft_setup(P));
   }
@@ -909,6 +917,16 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
   const int bits = bits_of(T);
   const int code_bits = code_sort_ok(P) && bits_of(TG) + kGCodeBits <= 31 ? kGCodeBits : 0;
   const int gbits = bits_of(TG) + code_bits;
+  // buffers grow on demand, if need be into the room of the rows (without them
+  // the plan grids from coil rows)
+  auto grow = [&](auto** p, int64_t n) {
+    int rc = dev_alloc(p, (size_t)n);
+    if (rc == MRN_OK || !P->d_rows) return rc;
+    cudaGetLastError();
+    cudaFree(P->d_rows);
+    P->d_rows = nullptr;
+    return dev_alloc(p, (size_t)n);
+  };
   P->traj_set = false;
   P->code_sorted = code_bits > 0;
   window_taps(P);
@@ -961,11 +979,12 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
   // 2. gridding entry buffers grow on demand
   const int64_t capE = std::max<int64_t>(E, 1);
   if (P->cap_entries < capE) {
-    RK(dev_alloc(&P->d_key_b, (size_t)capE));
-    RK(dev_alloc(&P->d_val_b, (size_t)capE));
-    RK(dev_alloc(&P->d_key_g, (size_t)capE));
-    RK(dev_alloc(&P->d_perm_g, (size_t)capE));
-    RK(dev_alloc(&P->d_coord_g, (size_t)capE));
+    P->cap_entries = 0;  // until all of them are there
+    RK(grow(&P->d_key_b, capE));
+    RK(grow(&P->d_val_b, capE));
+    RK(grow(&P->d_key_g, capE));
+    RK(grow(&P->d_perm_g, capE));
+    RK(grow(&P->d_coord_g, capE));
     P->cap_entries = capE;
   }
 
@@ -1021,25 +1040,29 @@ int mrn_plan_set_traj(mrn_plan* P, const float* trj, void* stream_) {
   const int64_t max_items_g = (int64_t)TG + full + 1;
   if (max_items_i >= (int64_t)INT32_MAX || max_items_g >= (int64_t)INT32_MAX) return MRN_ERR_UNSUPPORTED;
   if (P->cap_items_i < max_items_i) {
-    RK(dev_alloc(&P->d_items_i, (size_t)max_items_i));
+    P->cap_items_i = 0;
+    RK(grow(&P->d_items_i, max_items_i));
     P->cap_items_i = max_items_i;
   }
   if (P->cap_items_g < max_items_g) {
-    RK(dev_alloc(&P->d_items_g, (size_t)max_items_g));
+    P->cap_items_g = 0;
+    RK(grow(&P->d_items_g, max_items_g));
     P->cap_items_g = max_items_g;
   }
   const int64_t max_items = std::max(max_items_i, max_items_g);
   if (P->cap_sort < max_items) {
-    RK(dev_alloc(&P->d_items_tmp, (size_t)max_items));
+    P->cap_sort = 0;
+    RK(grow(&P->d_items_tmp, max_items));
     for (int k = 0; k < 2; ++k) {
-      RK(dev_alloc(&P->d_sort_key[k], (size_t)max_items));
-      RK(dev_alloc(&P->d_sort_idx[k], (size_t)max_items));
+      RK(grow(&P->d_sort_key[k], max_items));
+      RK(grow(&P->d_sort_idx[k], max_items));
     }
     P->cap_sort = max_items;
   }
   const int64_t part_elems = max_slots * (int64_t)P->max_coil * grid_tile_cells(P);
   if (P->cap_part < part_elems) {
-    RK(dev_alloc(&P->d_part, (size_t)part_elems));
+    P->cap_part = 0;
+    RK(grow(&P->d_part, part_elems));
     P->cap_part = part_elems;
   }
   {
