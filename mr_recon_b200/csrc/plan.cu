@@ -294,7 +294,7 @@ __host__ __device__ static int grid_chunk_of(int ndim, int sm_count, int64_t ent
   if (ndim == 1) return 1024;
   const int64_t lo = ndim == 2 ? 96 : 512, hi = ndim == 2 ? 256 : 4096;
   const int64_t share = entries / ((ndim == 2 ? 6 : 4) * (int64_t)sm_count);
-  const int64_t c = (share + 31) / 32 * 32;
+  const int64_t step = ndim == 2 ? 64 : 32, c = (share + step - 1) / step * step;
   return (int)(c < lo ? lo : (c > hi ? hi : c));
 }
 
