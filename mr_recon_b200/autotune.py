@@ -33,14 +33,15 @@ def clear_cache() -> None:
 
 
 def default_candidates(ndim: int) -> dict:
-    """Candidate values per option. 2D gridding tiles stay at most 8 cells
-    so the register-tile gridding kernel applies."""
+    """Candidate values per option, the defaults of every sample count among
+    them. 2D gridding tiles stay at most 8 cells so the register-tile gridding
+    kernel applies."""
     if ndim == 2:
         return {"interp_tile": [8, 10, 12], "interp_chunk": [128, 256],
-                "grid_tile": [6, 8], "grid_chunk": [128, 192, 256, 384]}
+                "grid_tile": [6, 8], "grid_chunk": [64, 96, 128, 192, 256, 384]}
     if ndim == 3:
         return {"interp_tile": [4, 5, 6], "interp_chunk": [256, 1024],
-                "grid_tile": [6, 8], "grid_chunk": [1024, 2048, 4096]}
+                "grid_tile": [6, 8], "grid_chunk": [512, 1024, 2048, 4096]}
     return {"interp_tile": [128, 256], "interp_chunk": [512, 1024],
             "grid_tile": [128, 256], "grid_chunk": [512, 1024]}
 
