@@ -45,14 +45,13 @@ NINTL, NSAMP = 48, 2048
 OS, W = 1.25, 6
 WORKLOAD = "2D multi-coil KB NUFFT fwd+adj: 256x256 c64, 32 coils, VD spiral 48x2048, os 1.25, W 6"
 HOST_AHEAD_S = 0.4e-3  # device-side wait before each timed step: longer than the host's enqueue of one step
-# DRAM bytes (read + write) per launch of each tile kernel on this workload,
-# from one ncu capture of the kernels named in TRAFFIC_SOURCE (ncu cannot run
-# inside the timed program, so the figure is carried here and labelled).
-GRID_TRAFFIC_BYTES = 30_618_624 + 2_219_264
-INTERP_TRAFFIC_BYTES = 26_141_440 + 982_272
-TRAFFIC_SOURCE = ("ncu --set full capture of k_grid_reg<7,1> (write-back staged through shared memory) "
-                  "and k_interp_reg<2,7,1> on this workload (dram__bytes_read.sum + dram__bytes_write.sum "
-                  "per launch)")
+# DRAM bytes (read + write) of the tile kernels on this workload, from one ncu
+# capture of the kernels named in TRAFFIC_SOURCE (ncu cannot run inside the
+# timed program, so the figure is carried here and labelled).
+GRID_TRAFFIC_BYTES = 25_173_760 + 32_379_392 + 10_750_976
+INTERP_TRAFFIC_BYTES = 24_910_336
+TRAFFIC_SOURCE = ("ncu capture of k_rows, k_grid_rows<2,7,32> and k_reduce_split<2> (gridding) and "
+                  "k_interp_tile<7,2> on this workload (dram__bytes_read.sum + dram__bytes_write.sum, cold L2)")
 CG_FIXTURE = os.path.join(ROOT, "tests", "golden", "cg_config2.npz")
 # Speed of the oracle port relative to the reference's own CPU path
 # (triton_nufft on CPU tensors, its torch fallback) on this workload: both

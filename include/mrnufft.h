@@ -131,7 +131,8 @@ int mrn_plan_fft_kind(const mrn_plan* plan);
  * group of fewer lanes than 32 splits a warp into entry streams whose partial
  * tiles are added at the end, so the summation order depends on it; a
  * one-slice plan given the lane count of a larger uneven plan (the lanes its
- * widest slice needs) adds every cell in the same order as that plan. */
+ * widest slice needs) adds every cell in the same order as that plan (work
+ * items and windows depend on the slice alone). */
 #define MRN_OPT_GRID_LANES 10
 /* MRN_OPT_ENTRY_MAJOR (default 1): mrn_sense_normal keeps its samples
  * sample-major (the coils of a sample side by side) between the interpolation
@@ -141,12 +142,13 @@ int mrn_plan_fft_kind(const mrn_plan* plan);
 /* MRN_OPT_NATIVE_FFT (default 1): the FFT stage as the library's own passes
  * (one per axis, Stockham, radices up to 20) with the apodize /
  * zero-pad folded into the first forward pass and the crop / deapodize into
- * the last adjoint pass, the zero-padded lines skipped; 2D and 3D groups of
- * one image and grid size whose lengths are products of 2, 3 and 5 of at most
- * 1024, from 96 points also with factors 7 to 19, and (chirp convolution, plans
- * of several grid sizes or large grids) any other length to 512. The Toeplitz
- * grids follow the value at the time the kernels are set (direct lengths only).
- * 0 (or any other plan) uses cuFFT between separate
+ * the last adjoint pass, the zero-padded lines skipped; for 2D and 3D slices,
+ * by their own grid and coils alone: lengths of products of 2, 3 and 5 of at most
+ * 1024, from 96 points also two factors of up to 20 with primes 7 to 19, and (chirp
+ * convolution, from 0.7 M grid points or for slabs of at most 20) lengths to 512 with a prime
+ * factor above 31. The Toeplitz grids follow the value at the time the kernels
+ * are set (products of factors up to 19, each slice by its own padded sizes).
+ * 0 (or any other slice) uses cuFFT between separate
  * pad and crop kernels. The two agree to float32 rounding, not bitwise. */
 #define MRN_OPT_NATIVE_FFT 12
 int mrn_plan_set_option(mrn_plan* plan, int option, int value);

@@ -31,8 +31,8 @@
 // 2-3-5 product up to 225 and most up to 400) crosses shared memory once. The
 // passes are bound by HBM in 3D and by latency on L2-resident 2D grids.
 // Measured (192^3 image, 240^3 grid, 16 coils): the three forward passes take
-// 1.93 ms (7.8 GB through HBM: 62% of the copy bandwidth), the inverse ones
-// 1.76; passes over coil planes that crossed shared memory before the first,
+// 1.87 ms (7.8 GB through HBM: 64% of the copy bandwidth), the inverse ones
+// 1.60; passes over coil planes that crossed shared memory before the first,
 // between all and after the last stage took 2.61 and 2.48 ms.
 #include <algorithm>
 #include <cmath>
@@ -50,7 +50,10 @@ namespace {
 constexpr int kFfxMaxRadix = 20;
 
 constexpr int kRadices[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 19, 20};
-constexpr int kMidMax = 12;  // largest radix of a middle stage
+// Largest radix of a middle stage; no length to 1024 needs one above 10, but without
+// the instances for 11 and 12 the passes of 512 points compile to 147 us a
+// Toeplitz normal (256^2, 32 coils) against 143.
+constexpr int kMidMax = 12;
 
 // Radices of n: two stages with the smallest larger radix where one exists,
 // else three, else four (first and last up to 20, the middle ones up to 12);
